@@ -118,6 +118,13 @@ enum {
 /* Most heavy probe keys a plan can name. */
 #define PJ_MAX_HEAVY 256
 
+/* pj_plan.flags: a planner made this plan for the join's sizes (pj_plan_exact,
+ * pj_plan_learned), so a join whose build side's hash table stays in L2 may
+ * skip the partitions; the pairs are those of any plan.  A default plan that
+ * the caller did not change counts as such without the flag; a plan
+ * without it runs as written. */
+#define PJ_PLAN_FLAG_AUTO 1
+
 /* Execution plan.  pj_plan_default() fills it from the sizes alone,
  * pj_plan_exact() from device histograms.  Passing NULL to pj_inner_join()
  * uses pj_plan_default(). */
@@ -140,7 +147,7 @@ typedef struct pj_plan {
     int32_t scatter_ctas_per_sm;/* scatter chunks per SM */
     int32_t hist_split;         /* histogram CTAs per scatter chunk */
     float max_fill;             /* OPEN: target fill (the reference's HASH_TABLE_OCC = 0.5) */
-    int32_t flags;              /* reserved, 0 */
+    int32_t flags;              /* PJ_PLAN_FLAG_* */
     int32_t n_heavy;            /* heavy probe keys below (0: no heavy-key path) */
     int32_t heavy_reserved;     /* 0 */
     int64_t heavy_keys[PJ_MAX_HEAVY]; /* probe keys matched outside the partitions, by a

@@ -12,6 +12,7 @@
 
 #include "../../include/pj.h"
 #include "pj_device.cuh"
+#include "pj_global.cuh"
 #include "pj_internal.h"
 #include "pj_join.cuh"
 #include "pj_partition.cuh"
@@ -41,6 +42,8 @@ constexpr int HEAVY_SAMPLES = 1 << 16;     // probe keys the planner samples
 constexpr int HEAVY_MIN_SAMPLES = 32;      // a heavy key holds >= 1/2048 of the sample
 constexpr int64_t HEAVY_MIN_PROBE = 1 << 20;  // smaller probe sides: no heavy-key path
 constexpr double HEAVY_MIN_SHARE = 0.5;       // share of the probe rows the heavy keys must hold
+constexpr int64_t GLOBAL_MAX_BUILD = 1 << 22;     // build rows of a join by one table in L2
+constexpr int64_t GLOBAL_SPARSE_BUILD = 1 << 20;  // up to here its table has four slots a row
 constexpr size_t LEARN_BYTES = 4096;          // features, activations and scores of the learned planner
 
 struct DevInfo {
@@ -776,7 +779,7 @@ pj_status partition_column(const K* keys, int64_t n, const pj_plan* p, const Lay
     E.mark(stage0, st);
     if ((s = launch_hist<K>(keys, n, chunk, items, p->hist_split, f, P1, counts, tot, st, hc)) != PJ_OK) return s;
     E.mark(stage0 + 1, st);
-    if ((s = launch_scan<uint32_t>(counts, static_cast<int64_t>(P1) * items, static_cast<uint32_t>(p->wc_tuples), off,
+    if ((s = launch_scan(counts, static_cast<int64_t>(P1) * items, static_cast<uint32_t>(p->wc_tuples), off,
                                    tiles, ctr + (side == 0 ? CTR_BTILE : CTR_PTILE), status, st)) != PJ_OK)
         return s;
     E.mark(stage0 + 2, st);
@@ -826,7 +829,7 @@ pj_status partition_pass2(const pj_plan* p, const Layout& L, int side, uint8_t* 
     PJ_CUDA(cudaGetLastError());
     pj_status s;
     const int W2 = pass2_wc(static_cast<int>(sizeof(K)), p);
-    if ((s = launch_scan<uint32_t>(counts, static_cast<int64_t>(P2) * n_items, static_cast<uint32_t>(W2), off, tiles,
+    if ((s = launch_scan(counts, static_cast<int64_t>(P2) * n_items, static_cast<uint32_t>(W2), off, tiles,
                                    ctr + (side == 0 ? CTR_BTILE2 : CTR_PTILE2), status, st)) != PJ_OK)
         return s;
     switch (W2) {
@@ -839,6 +842,121 @@ pj_status partition_pass2(const pj_plan* p, const Layout& L, int side, uint8_t* 
     }
 }
 
+// Payload columns of the pairs written (no-op without them).
+pj_status launch_payload(const pj_join_desc* d, const int32_t* out_b, const int32_t* out_p, int64_t capacity,
+                         const int64_t* count, void* pay_b, void* pay_p, cudaStream_t st)
+{
+    if (!out_b || !(pay_b || pay_p) || d->payload_bytes <= 0) return PJ_OK;
+    const unsigned grid = static_cast<unsigned>(sm_count()) * 8;
+    const auto* cnt = reinterpret_cast<const unsigned long long*>(count);
+    if (d->payload_bytes == 4)
+        gather_payload_kernel<int32_t><<<grid, 256, 0, st>>>(
+            out_b, out_p, static_cast<const int32_t*>(d->build_payload), static_cast<const int32_t*>(d->probe_payload),
+            static_cast<int32_t*>(pay_b), static_cast<int32_t*>(pay_p), cnt, capacity);
+    else
+        gather_payload_kernel<int64_t><<<grid, 256, 0, st>>>(
+            out_b, out_p, static_cast<const int64_t*>(d->build_payload), static_cast<const int64_t*>(d->probe_payload),
+            static_cast<int64_t*>(pay_b), static_cast<int64_t*>(pay_p), cnt, capacity);
+    PJ_CUDA(cudaGetLastError());
+    return PJ_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Joins by one table in L2 (pj_global.cuh).
+struct GlobalPlan {
+    bool use = false;
+    uint32_t nb = 0;          // buckets
+    size_t zeroed = 0;        // workspace bytes to clear, from 0
+    size_t table = 0;         // unique: buckets; repeated keys: bucket counts
+    size_t range = 0, entries = 0;  // repeated keys
+};
+
+// Whether a planner's schedule (not one a caller wrote) is asked for: the
+// default plan unchanged, or PJ_PLAN_FLAG_AUTO.
+bool planner_made(const pj_join_desc* d, const pj_plan* p)
+{
+    if (p->flags & PJ_PLAN_FLAG_AUTO) return true;
+    pj_plan q;
+    return pj_plan_default(d, &q) == PJ_OK && std::memcmp(p, &q, sizeof(q)) == 0;
+}
+
+// The global table lives in the bytes that the partitioned layout has
+// anyway, so no workspace grows; a join whose table does not fit them
+// (many more build than probe rows) is partitioned.
+GlobalPlan global_plan(const pj_join_desc* d, const pj_plan* p, const Layout& L)
+{
+    GlobalPlan g;
+    const int64_t n = d->n_build;
+    if (n < 1 || d->n_probe < 1 || n > GLOBAL_MAX_BUILD || !planner_made(d, p)) return g;
+    const size_t o = align_up(L.counters + 4 * 8, 256);
+    g.table = o;
+    if (d->unique_build_keys) {
+        // four 8-byte slots (4-byte keys) or eight 4-byte slots (8-byte keys)
+        // a bucket.  One row a bucket while the table stays small; beyond, two
+        // rows (three for 8-byte keys: 14 % of four-slot buckets are full at
+        // two, 1 % of eight-slot ones at three) to keep it and the build keys
+        // in L2.
+        const int64_t per = n <= GLOBAL_SPARSE_BUILD ? 1 : d->key_bytes == 4 ? 2 : 3;
+        const int64_t slots = d->key_bytes == 4 ? 4 : 8;
+        const int64_t want = std::max<int64_t>(8, (n + per - 1) / per);
+        const int64_t fit = static_cast<int64_t>((L.total - o) / 32);
+        g.nb = static_cast<uint32_t>(std::min(want, fit));
+        g.zeroed = o + 32 * static_cast<size_t>(g.nb);
+        g.use = slots * static_cast<int64_t>(g.nb) >= n + n / 2 + 8;
+        return g;
+    }
+    g.nb = static_cast<uint32_t>(std::max<int64_t>(8, n));
+    g.zeroed = align_up(o + 4 * static_cast<size_t>(g.nb), 256);
+    g.range = g.zeroed;
+    g.entries = align_up(g.range + 8 * static_cast<size_t>(g.nb), 256);
+    g.use = g.entries + 8 * static_cast<size_t>(n) <= L.total;
+    return g;
+}
+
+template <typename K>
+pj_status run_global(const pj_join_desc* d, const GlobalPlan& g, const Layout& L, uint8_t* ws, int32_t* out_b,
+                     int32_t* out_p, int64_t capacity, int64_t* count, cudaStream_t st, const StageEvents& E)
+{
+    uint32_t* status = reinterpret_cast<uint32_t*>(ws + L.status);
+    const K* bk = static_cast<const K*>(d->build_keys);
+    const K* pk = static_cast<const K*>(d->probe_keys);
+    const uint32_t nb = static_cast<uint32_t>(d->n_build), np = static_cast<uint32_t>(d->n_probe);
+    const unsigned bgrid = (nb + GT_THREADS - 1) / GT_THREADS, pgrid = (np + GT_TILE - 1) / GT_TILE;
+    auto* cnt = reinterpret_cast<unsigned long long*>(count);
+    const GlobalOut o{out_b, out_p, capacity, cnt, status};
+    for (int i = PJ_STAGE_BUILD_HIST; i <= PJ_STAGE_BUILD_SCATTER; ++i) E.mark(i, st);
+    PJ_CUDA(cudaMemsetAsync(ws, 0, g.zeroed, st));
+    if (d->unique_build_keys) {
+        auto* table = reinterpret_cast<uint32_t*>(ws + g.table);
+        gt_build_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, table, g.nb, cnt, status);
+        PJ_CUDA(cudaGetLastError());
+        for (int i = PJ_STAGE_BUILD_PASS2; i <= PJ_STAGE_JOIN; ++i) E.mark(i, st);
+        // several steps a CTA once they fill every SM twice over
+        const unsigned sgrid = (pgrid + GT_STEPS - 1) / GT_STEPS;
+        if (sgrid >= 12u * static_cast<unsigned>(sm_count()))
+            gt_probe_kernel<K, GT_STEPS><<<sgrid, GT_THREADS, 0, st>>>(pk, np, bk, table, g.nb, o);
+        else
+            gt_probe_kernel<K, 1><<<pgrid, GT_THREADS, 0, st>>>(pk, np, bk, table, g.nb, o);
+    } else {
+        auto* counts = reinterpret_cast<uint32_t*>(ws + g.table);
+        auto* range = reinterpret_cast<uint2*>(ws + g.range);
+        auto* entries = reinterpret_cast<uint2*>(ws + g.entries);
+        gt_count_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, counts, g.nb, cnt);
+        PJ_CUDA(cudaGetLastError());
+        // (the counter block's words double as the 64-bit entry cursor)
+        auto* cursor = reinterpret_cast<unsigned long long*>(ws + L.counters);
+        gt_alloc_kernel<<<(g.nb + GT_THREADS * GT_ALLOC - 1) / (GT_THREADS * GT_ALLOC), GT_THREADS, 0, st>>>(
+            counts, g.nb, range, cursor);
+        PJ_CUDA(cudaGetLastError());
+        gt_place_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, range, g.nb, entries);
+        PJ_CUDA(cudaGetLastError());
+        for (int i = PJ_STAGE_BUILD_PASS2; i <= PJ_STAGE_JOIN; ++i) E.mark(i, st);
+        gt_probe_multi_kernel<K><<<pgrid, GT_THREADS, 0, st>>>(pk, np, bk, range, g.nb, entries, o);
+    }
+    PJ_CUDA(cudaGetLastError());
+    return PJ_OK;
+}
+
 template <typename K>
 pj_status run_join(const pj_join_desc* d, const pj_plan* p, const Layout& L, uint8_t* ws, int32_t* out_b,
                    int32_t* out_p, int64_t capacity, int64_t* count, void* pay_b, void* pay_p, cudaStream_t st,
@@ -846,6 +964,13 @@ pj_status run_join(const pj_join_desc* d, const pj_plan* p, const Layout& L, uin
 {
     uint32_t* status = reinterpret_cast<uint32_t*>(ws + L.status);
     uint32_t* ctr = reinterpret_cast<uint32_t*>(ws + L.counters);
+    const GlobalPlan g = global_plan(d, p, L);
+    if (g.use) {
+        pj_status s = run_global<K>(d, g, L, ws, out_b, out_p, capacity, count, st, E);
+        if (s == PJ_OK) s = launch_payload(d, out_b, out_p, capacity, count, pay_b, pay_p, st);
+        E.mark(PJ_STAGE_TOTAL, st);
+        return s;
+    }
     PJ_CUDA(cudaMemsetAsync(ws, 0, L.ctrl_end, st));
     PJ_CUDA(cudaMemsetAsync(count, 0, sizeof(int64_t), st));
     if (d->n_build == 0 || d->n_probe == 0) {
@@ -907,7 +1032,7 @@ pj_status run_join(const pj_join_desc* d, const pj_plan* p, const Layout& L, uin
         hash_split ? cap_tuples : position_chunk, p->probe_chunk, hash_split ? 1 : 0, MAX_SPLIT_LOG2,
         reinterpret_cast<int32_t*>(ws + L.split), reinterpret_cast<int64_t*>(ws + L.items), status, nullptr);
     PJ_CUDA(cudaGetLastError());
-    if ((s = launch_scan<int64_t>(reinterpret_cast<int64_t*>(ws + L.items), L.P, 1u,
+    if ((s = launch_scan(reinterpret_cast<int64_t*>(ws + L.items), L.P, 1u,
                                   reinterpret_cast<int64_t*>(ws + L.item_off), reinterpret_cast<uint64_t*>(ws + L.i_tiles),
                                   ctr + CTR_ITILE, status, st)) != PJ_OK)
         return s;
@@ -950,19 +1075,7 @@ pj_status run_join(const pj_join_desc* d, const pj_plan* p, const Layout& L, uin
     a.base_count = heavy_total;
     E.mark(PJ_STAGE_JOIN, st);
     s = launch_join<K>(a, p->table_mode, d->unique_build_keys != 0, hash_split, p->slot_mode == PJ_SLOT_REF, st);
-    if (s == PJ_OK && out_b && (pay_b || pay_p) && d->payload_bytes > 0) {
-        const unsigned grid = static_cast<unsigned>(sm_count()) * 8;
-        const auto* cnt = reinterpret_cast<const unsigned long long*>(count);
-        if (d->payload_bytes == 4)
-            gather_payload_kernel<int32_t><<<grid, 256, 0, st>>>(
-                out_b, out_p, static_cast<const int32_t*>(d->build_payload), static_cast<const int32_t*>(d->probe_payload),
-                static_cast<int32_t*>(pay_b), static_cast<int32_t*>(pay_p), cnt, capacity);
-        else
-            gather_payload_kernel<int64_t><<<grid, 256, 0, st>>>(
-                out_b, out_p, static_cast<const int64_t*>(d->build_payload), static_cast<const int64_t*>(d->probe_payload),
-                static_cast<int64_t*>(pay_b), static_cast<int64_t*>(pay_p), cnt, capacity);
-        PJ_CUDA(cudaGetLastError());
-    }
+    if (s == PJ_OK) s = launch_payload(d, out_b, out_p, capacity, count, pay_b, pay_p, st);
     E.mark(PJ_STAGE_TOTAL, st);
     return s;
 }
@@ -1251,7 +1364,7 @@ pj_status pj_diag_scan_timeout(const pj_join_desc* d, const pj_plan* plan, void*
     uint8_t* w = static_cast<uint8_t*>(ws);
     PJ_CUDA(cudaMemsetAsync(w, 0, L.ctrl_end, st));  // as a join starts: zero counts, tile states, status
     uint32_t* ctr = reinterpret_cast<uint32_t*>(w + L.counters);
-    return launch_scan<uint32_t>(reinterpret_cast<const uint32_t*>(w + L.b_counts), m, 1u,
+    return launch_scan(reinterpret_cast<const uint32_t*>(w + L.b_counts), m, 1u,
                                  reinterpret_cast<int64_t*>(w + L.b_off), reinterpret_cast<uint64_t*>(w + L.b_tiles),
                                  ctr + CTR_BTILE, reinterpret_cast<uint32_t*>(w + L.status), st,
                                  ScanWait{withhold_tile, spin_limit});
@@ -1470,6 +1583,7 @@ pj_status pj_plan_exact(const pj_join_desc* d, void* ws, size_t ws_bytes, pj_pla
     // Hash splits cannot separate repeated keys: a partition beyond what
     // 2^MAX_SPLIT_LOG2 tables hold (duplicates) takes the position split.
     if (mx_plan > cap * (int64_t(1) << MAX_SPLIT_LOG2) / 2) p.split_mode = PJ_SPLIT_POSITION;
+    if (d->n_build <= GLOBAL_MAX_BUILD) p.flags = PJ_PLAN_FLAG_AUTO;
     *plan = p;
     return PJ_OK;
 }
@@ -1613,7 +1727,15 @@ pj_status pj_plan_learned(const pj_join_desc* d, const float* params, void* ws, 
     std::sort(order, order + PJ_PLAN_CANDIDATES, [&](int a, int b) { return out[a] < out[b]; });
     for (int c : order) {
         if (c == PJ_PLAN_CANDIDATE_EXACT) return pj_plan_exact(d, ws, ws_bytes, plan, stream);
-        if (pj_plan_candidate(d, c, &heavy, plan) == PJ_OK) return PJ_OK;
+        if (pj_plan_candidate(d, c, &heavy, plan) == PJ_OK) {
+            // (a COMPACT choice that the sizes already rule out runs as written: its overflow is the caller's
+            // signal to fall back)
+            const double m = static_cast<double>(d->n_build) / static_cast<double>(int64_t(1) << plan->bits1);
+            if (d->n_build <= GLOBAL_MAX_BUILD &&
+                (plan->table_mode != PJ_TABLE_COMPACT || m + 4.0 * std::sqrt(m) <= static_cast<double>(COMPACT_RANGE)))
+                plan->flags = PJ_PLAN_FLAG_AUTO;
+            return PJ_OK;
+        }
     }
     return pj_plan_default(d, plan);
 }
@@ -1649,7 +1771,7 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
     hist_seg_kernel<K><<<static_cast<unsigned>(n_items) * 2, HIST_THREADS, hsmem, st>>>(items, 2, counts, totals);
     PJ_CUDA(cudaGetLastError());
     pj_status s;
-    if ((s = launch_scan<uint32_t>(counts, lb.n_counts, static_cast<uint32_t>(lb.W), off,
+    if ((s = launch_scan(counts, lb.n_counts, static_cast<uint32_t>(lb.W), off,
                                    reinterpret_cast<uint64_t*>(w + lb.o_tiles), ctr + CTR_BTILE, status, st)) != PJ_OK)
         return s;
     constexpr int VT = sizeof(K) == 4 ? 4 : 2;
@@ -1682,7 +1804,7 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
         hash_split ? 1 : 0, MAX_SPLIT_LOG2, reinterpret_cast<int32_t*>(w + lb.o_split),
         reinterpret_cast<int64_t*>(w + lb.o_jitems), status, parts);
     PJ_CUDA(cudaGetLastError());
-    if ((s = launch_scan<int64_t>(reinterpret_cast<int64_t*>(w + lb.o_jitems), lb.G, 1u,
+    if ((s = launch_scan(reinterpret_cast<int64_t*>(w + lb.o_jitems), lb.G, 1u,
                                   reinterpret_cast<int64_t*>(w + lb.o_item_off),
                                   reinterpret_cast<uint64_t*>(w + lb.o_itiles), ctr + CTR_ITILE, status, st)) != PJ_OK)
         return s;
