@@ -44,6 +44,7 @@ constexpr int64_t HEAVY_MIN_PROBE = 1 << 20;  // smaller probe sides: no heavy-k
 constexpr double HEAVY_MIN_SHARE = 0.5;       // share of the probe rows the heavy keys must hold
 constexpr int64_t GLOBAL_MAX_BUILD = 1 << 22;     // build rows of a join by one table in L2
 constexpr int64_t GLOBAL_SPARSE_BUILD = 1 << 20;  // up to here its table has four slots a row
+constexpr int64_t GROUP_BYTES = int64_t(256) << 20;  // tuples of one item group (pj_partition.cuh)
 constexpr size_t LEARN_BYTES = 4096;          // features, activations and scores of the learned planner
 
 struct DevInfo {
@@ -354,6 +355,7 @@ struct Layout {
     size_t b_tuples2 = 0, p_tuples2 = 0;
     int64_t b_tiles2_n = 0, p_tiles2_n = 0;
     int b_items = 1, p_items = 1;
+    int b_ipg = 1, p_ipg = 1, b_groups = 1, p_groups = 1;  // first-pass items per group, groups
     int64_t b_chunk = 16, p_chunk = 16;
     int64_t b_cap = 0, p_cap = 0;  // tuples
     int64_t max_items = 0;
@@ -381,7 +383,19 @@ int scatter_items(const pj_plan* p) { return sm_count() * std::max(1, p->scatter
 
 int64_t part_capacity(int64_t n, int P, int items, int W) { return n + static_cast<int64_t>(items) * P * (W - 1) + W; }
 
-Layout make_layout(const pj_join_desc* d, const pj_plan* p)
+// Items per group (pj_partition.cuh) of a column of n_items chunks: groups of
+// at most GROUP_BYTES of tuples, at most MAX_GROUPS of them; one group while
+// the column is not much larger.
+int items_per_group(int n_items, int64_t chunk, int key_bytes)
+{
+    const int64_t bytes = chunk * tuple_words(key_bytes) * 4;
+    if (bytes * n_items <= 2 * GROUP_BYTES) return n_items;
+    const int64_t fit = std::max<int64_t>(1, GROUP_BYTES / bytes);
+    return static_cast<int>(std::max<int64_t>(fit, (n_items + MAX_GROUPS - 1) / MAX_GROUPS));
+}
+
+// grouped = false: partitions contiguous (pj_partition's result).
+Layout make_layout(const pj_join_desc* d, const pj_plan* p, bool grouped = true)
 {
     Layout L;
     const bool two = p->passes == 2;
@@ -401,7 +415,20 @@ Layout make_layout(const pj_join_desc* d, const pj_plan* p)
     }
     const int64_t m2 = static_cast<int64_t>(L.P) * L.C;  // second-pass segments per side
     L.b_tiles2_n = L.p_tiles2_n = two ? (m2 + SCAN_TILE - 1) / SCAN_TILE + 1 : 0;
-    const int64_t mb = static_cast<int64_t>(L.P1) * L.b_items, mp = static_cast<int64_t>(L.P1) * L.p_items;
+    L.b_ipg = L.b_items;
+    L.p_ipg = L.p_items;
+    // Groups where the join walks ranges by position in the partition: not for
+    // a second pass, COMPACT entries (which index the build range) or OPEN tables,
+    // nor for half-sector groups' own scatter.
+    if (grouped && !two && (p->table_mode == PJ_TABLE_BUCKET || p->table_mode == PJ_TABLE_EXACT) &&
+        sector_wc(d->key_bytes, p->wc_tuples)) {
+        L.b_ipg = items_per_group(L.b_items, L.b_chunk, d->key_bytes);
+        L.p_ipg = items_per_group(L.p_items, L.p_chunk, d->key_bytes);
+    }
+    L.b_groups = (L.b_items + L.b_ipg - 1) / L.b_ipg;
+    L.p_groups = (L.p_items + L.p_ipg - 1) / L.p_ipg;
+    const int64_t mb = static_cast<int64_t>(L.P1) * L.b_groups * L.b_ipg;
+    const int64_t mp = static_cast<int64_t>(L.P1) * L.p_groups * L.p_ipg;
     L.b_tiles_n = (mb + SCAN_TILE - 1) / SCAN_TILE + 1;
     L.p_tiles_n = (mp + SCAN_TILE - 1) / SCAN_TILE + 1;
     L.i_tiles_n = (L.P + SCAN_TILE - 1) / SCAN_TILE + 1;
@@ -614,7 +641,7 @@ struct HeavyCtx {
 };
 
 template <typename K, bool HASHD, bool HEAVY>
-pj_status launch_hist_t(const K* keys, int64_t n, int64_t chunk, int items, int hsplit, DigitFn f, int P,
+pj_status launch_hist_t(const K* keys, int64_t n, int64_t chunk, int items, int hsplit, DigitFn f, int P, int ipg,
                         uint32_t* counts, int32_t* totals, const HeavyCtx& hc, cudaStream_t st)
 {
     const size_t smem = 4 * static_cast<size_t>((P + 3) & ~3) + (HEAVY ? HeavyTable::BYTES : 0);
@@ -622,22 +649,22 @@ pj_status launch_hist_t(const K* keys, int64_t n, int64_t chunk, int items, int 
     PJ_CUDA(set_smem(kern, smem));
     typename HeavyArg<HEAVY>::type h{};
     if constexpr (HEAVY) h = *hc.hs;
-    kern<<<items * hsplit, HIST_THREADS, smem, st>>>(keys, n, chunk, items, hsplit, f, P, counts, totals, h, hc.out);
+    kern<<<items * hsplit, HIST_THREADS, smem, st>>>(keys, n, chunk, items, hsplit, f, P, ipg, counts, totals, h, hc.out);
     PJ_CUDA(cudaGetLastError());
     return PJ_OK;
 }
 
 // hc.hs: heavy probe keys to leave out (nullptr: none)
 template <typename K>
-pj_status launch_hist(const K* keys, int64_t n, int64_t chunk, int items, int hsplit, DigitFn f, int P,
+pj_status launch_hist(const K* keys, int64_t n, int64_t chunk, int items, int hsplit, DigitFn f, int P, int ipg,
                       uint32_t* counts, int32_t* totals, cudaStream_t st, const HeavyCtx& hc = HeavyCtx())
 {
     const bool hd = f.mode == PJ_DIGIT_HASH;
     if (hc.hs)
-        return hd ? launch_hist_t<K, true, true>(keys, n, chunk, items, hsplit, f, P, counts, totals, hc, st)
-                  : launch_hist_t<K, false, true>(keys, n, chunk, items, hsplit, f, P, counts, totals, hc, st);
-    return hd ? launch_hist_t<K, true, false>(keys, n, chunk, items, hsplit, f, P, counts, totals, hc, st)
-              : launch_hist_t<K, false, false>(keys, n, chunk, items, hsplit, f, P, counts, totals, hc, st);
+        return hd ? launch_hist_t<K, true, true>(keys, n, chunk, items, hsplit, f, P, ipg, counts, totals, hc, st)
+                  : launch_hist_t<K, false, true>(keys, n, chunk, items, hsplit, f, P, ipg, counts, totals, hc, st);
+    return hd ? launch_hist_t<K, true, false>(keys, n, chunk, items, hsplit, f, P, ipg, counts, totals, hc, st)
+              : launch_hist_t<K, false, false>(keys, n, chunk, items, hsplit, f, P, ipg, counts, totals, hc, st);
 }
 
 template <typename TIn>
@@ -652,55 +679,72 @@ pj_status launch_scan(const TIn* in, int64_t m, uint32_t round_to, int64_t* out,
     return PJ_OK;
 }
 
-template <typename K, int W, bool HASHD, bool HEAVY>
-pj_status launch_scatter_t(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P,
+// log2 of the tuples of a write-combining unit for P partitions: whole
+// sectors, at least W, and as large as about 128 KB over all partitions allow
+// (the fewer partitions, the more tuples of a round meet in one unit); -1
+// where units and cursors do not fit beside `extra` bytes.
+template <typename K>
+int unit_logf(int P, int W, int v, size_t extra)
+{
+    using U = WcUnits<K>;
+    int lf = U::LOG_CH;
+    while ((1 << lf) < W) ++lf;
+    if (lf > U::MAX_LOGF || U::bytes(P, lf, SC_THREADS, v) + extra > smem_limit()) return -1;
+    while (lf < U::MAX_LOGF && (static_cast<size_t>(P) << (lf + 1)) * U::TW * 4 <= (size_t(128) << 10) &&
+           U::bytes(P, lf + 1, SC_THREADS, v) + extra <= smem_limit())
+        ++lf;
+    return lf;
+}
+
+template <typename K, bool HASHD, bool HEAVY>
+pj_status launch_scatter_t(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P, int W, int ipg,
                            const int64_t* offsets, uint32_t* out, int64_t out_cap, uint32_t* status,
                            const HeavyCtx& hc, cudaStream_t st)
 {
-    auto* kern = scatter_keys_kernel<K, SC_THREADS, sc_v<K>(), W, HASHD, HEAVY>;
-    constexpr int TW = WcTraits<K, W>::TW;
-    const int cap = wc_cap(sizeof(K), W, P, SC_THREADS * sc_v<K>(), HEAVY ? HeavyTable::BYTES + 16 : 0);
-    const size_t smem = HEAVY ? heavy_table_offset(P, cap * TW) + HeavyTable::BYTES : scatter_smem(sizeof(K), cap, P);
-    PJ_CUDA(set_smem(kern, smem));
     typename HeavyArg<HEAVY>::type h{};
     if constexpr (HEAVY) h = *hc.hs;
-    kern<<<items, SC_THREADS, smem, st>>>(keys, n, chunk, items, f, P, cap, offsets, out,
-                                         static_cast<uint32_t>(std::min<int64_t>(out_cap, UINT32_MAX)), status, h,
-                                         hc.out);
-    PJ_CUDA(cudaGetLastError());
-    return PJ_OK;
-}
-
-template <typename K, int W>
-pj_status launch_scatter_w(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P,
-                           const int64_t* offsets, uint32_t* out, int64_t out_cap, uint32_t* status,
-                           const HeavyCtx& hc, cudaStream_t st)
-{
-    const bool hd = f.mode == PJ_DIGIT_HASH;
-    if (hc.hs)
-        return hd ? launch_scatter_t<K, W, true, true>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st)
-                  : launch_scatter_t<K, W, false, true>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st);
-    return hd ? launch_scatter_t<K, W, true, false>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st)
-              : launch_scatter_t<K, W, false, false>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st);
-}
-
-template <typename K>
-pj_status launch_scatter(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P, int W,
-                         const int64_t* offsets, uint32_t* out, int64_t out_cap, uint32_t* status, cudaStream_t st,
-                         const HeavyCtx& hc = HeavyCtx())
-{
-    if (W == 2) return launch_scatter_w<K, 2>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st);
-    if (W == 4) return launch_scatter_w<K, 4>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st);
-    if (W == 8) return launch_scatter_w<K, 8>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st);
-    if (W == 16) return launch_scatter_w<K, 16>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st);
-    if (W == 32) return launch_scatter_w<K, 32>(keys, n, chunk, items, f, P, offsets, out, out_cap, status, hc, st);
+    const uint32_t cap32 = static_cast<uint32_t>(std::min<int64_t>(out_cap, UINT32_MAX));
+    constexpr int V = sc_v<K>();
+    const int lf = unit_logf<K>(P, W, V, HEAVY ? HeavyTable::BYTES + 16 : 0);
+    if (lf >= 0 && chunk <= static_cast<int64_t>(WCU_COUNT)) {
+        auto* kern = scatter_keys_kernel<K, SC_THREADS, V, HASHD, HEAVY>;
+        const size_t smem = WcUnits<K>::bytes(P, lf, SC_THREADS, V) + (HEAVY ? HeavyTable::BYTES + 16 : 0);
+        PJ_CUDA(set_smem(kern, smem));
+        kern<<<items, SC_THREADS, smem, st>>>(keys, n, chunk, items, f, P, lf, W, ipg, offsets, out, cap32, status, h, hc.out);
+        PJ_CUDA(cudaGetLastError());
+        return PJ_OK;
+    }
+    if constexpr (sizeof(K) == 4) {  // 8192 partitions of half-sector groups
+        if (W != 2 || ipg != items) return PJ_ERR_INVALID;
+        auto* kern = scatter_rounds_kernel<K, SC_THREADS, V, 2, HASHD, HEAVY>;
+        constexpr int TW = WcTraits<K, 2>::TW;
+        const int cap = wc_cap(sizeof(K), W, P, SC_THREADS * V, HEAVY ? HeavyTable::BYTES + 16 : 0);
+        const size_t smem = HEAVY ? heavy_table_offset(P, cap * TW) + HeavyTable::BYTES : scatter_smem(sizeof(K), cap, P);
+        PJ_CUDA(set_smem(kern, smem));
+        kern<<<items, SC_THREADS, smem, st>>>(keys, n, chunk, items, f, P, cap, offsets, out, cap32, status, h, hc.out);
+        PJ_CUDA(cudaGetLastError());
+        return PJ_OK;
+    }
     return PJ_ERR_INVALID;
 }
 
-template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF>
-pj_status launch_join_t(const JoinArgs& a, cudaStream_t st)
+template <typename K>
+pj_status launch_scatter(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P, int W, int ipg,
+                         const int64_t* offsets, uint32_t* out, int64_t out_cap, uint32_t* status, cudaStream_t st,
+                         const HeavyCtx& hc = HeavyCtx())
 {
-    auto* kern = join_kernel<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, JN_THREADS>;
+    const bool hd = f.mode == PJ_DIGIT_HASH;
+    if (hc.hs)
+        return hd ? launch_scatter_t<K, true, true>(keys, n, chunk, items, f, P, W, ipg, offsets, out, out_cap, status, hc, st)
+                  : launch_scatter_t<K, false, true>(keys, n, chunk, items, f, P, W, ipg, offsets, out, out_cap, status, hc, st);
+    return hd ? launch_scatter_t<K, true, false>(keys, n, chunk, items, f, P, W, ipg, offsets, out, out_cap, status, hc, st)
+              : launch_scatter_t<K, false, false>(keys, n, chunk, items, f, P, W, ipg, offsets, out, out_cap, status, hc, st);
+}
+
+template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF, int NG>
+pj_status launch_join_g(const JoinArgs& a, cudaStream_t st)
+{
+    auto* kern = join_kernel<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, JN_THREADS, NG>;
     const size_t smem = JoinSmem<K, TABLE>::bytes(a.cap, a.nb_log2);
     PJ_CUDA(set_smem(kern, smem));
     int per_sm = 0;
@@ -720,6 +764,15 @@ pj_status launch_join_t(const JoinArgs& a, cudaStream_t st)
         PJ_CUDA(cudaGetLastError());
     }
     return PJ_OK;
+}
+
+template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF>
+pj_status launch_join_t(const JoinArgs& a, cudaStream_t st)
+{
+    if constexpr (TABLE == TABLE_BUCKET || TABLE == TABLE_EXACT)
+        if (a.b_groups > 1 || a.p_groups > 1) return launch_join_g<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, MAX_GROUPS>(a, st);
+    if (a.b_groups != 1 || a.p_groups != 1) return PJ_ERR_INVALID;
+    return launch_join_g<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, 1>(a, st);
 }
 
 template <typename K, int TABLE>
@@ -767,6 +820,7 @@ pj_status partition_column(const K* keys, int64_t n, const pj_plan* p, const Lay
     const int P1 = L.P1;
     const int64_t chunk = side == 0 ? L.b_chunk : L.p_chunk;
     const int items = side == 0 ? L.b_items : L.p_items;
+    const int ipg = side == 0 ? L.b_ipg : L.p_ipg, groups = side == 0 ? L.b_groups : L.p_groups;
     uint32_t* status = reinterpret_cast<uint32_t*>(ws + L.status);
     uint32_t* ctr = reinterpret_cast<uint32_t*>(ws + L.counters);
     uint32_t* counts = reinterpret_cast<uint32_t*>(ws + (side == 0 ? L.b_counts : L.p_counts));
@@ -777,30 +831,31 @@ pj_status partition_column(const K* keys, int64_t n, const pj_plan* p, const Lay
     uint64_t* tiles = reinterpret_cast<uint64_t*>(ws + (side == 0 ? L.b_tiles : L.p_tiles));
     pj_status s;
     E.mark(stage0, st);
-    if ((s = launch_hist<K>(keys, n, chunk, items, p->hist_split, f, P1, counts, tot, st, hc)) != PJ_OK) return s;
+    if ((s = launch_hist<K>(keys, n, chunk, items, p->hist_split, f, P1, ipg, counts, tot, st, hc)) != PJ_OK) return s;
     E.mark(stage0 + 1, st);
-    if ((s = launch_scan(counts, static_cast<int64_t>(P1) * items, static_cast<uint32_t>(p->wc_tuples), off,
+    if ((s = launch_scan(counts, static_cast<int64_t>(P1) * groups * ipg, static_cast<uint32_t>(p->wc_tuples), off,
                                    tiles, ctr + (side == 0 ? CTR_BTILE : CTR_PTILE), status, st)) != PJ_OK)
         return s;
     E.mark(stage0 + 2, st);
-    return launch_scatter<K>(keys, n, chunk, items, f, P1, p->wc_tuples, off, tuples, cap, status, st, hc);
+    return launch_scatter<K>(keys, n, chunk, items, f, P1, p->wc_tuples, ipg, off, tuples, cap, status, st, hc);
 }
 
 // Second pass of a two-pass plan over one side's first-pass tuples:
 // histogram -> look-back scan -> scatter into the side's second tuple buffer.
 // The digit is the next bits2 hash bits below those the first pass used.
-template <typename K, int W>
-pj_status launch_scatter_tuples(const uint32_t* in, const Pass2Items& it, int n_items, DigitFn f, int P2,
+template <typename K>
+pj_status launch_scatter_tuples(const uint32_t* in, const Pass2Items& it, int n_items, DigitFn f, int P2, int W,
                                 const int64_t* off, uint32_t* out, int64_t cap, uint32_t* status, cudaStream_t st)
 {
     constexpr int VT = sizeof(K) == 4 ? 4 : 2;
-    auto* kern = scatter_tuples_kernel<K, SC_THREADS, VT, W>;
-    const int bcap = wc_cap(sizeof(K), W, P2, SC_THREADS * VT, 0);
-    const size_t smem = scatter_smem(sizeof(K), bcap, P2);
+    auto* kern = scatter_tuples_kernel<K, SC_THREADS, VT>;
+    const int lf = unit_logf<K>(P2, W, VT, 0);
+    if (lf < 0) return PJ_ERR_INVALID;
+    const size_t smem = WcUnits<K>::bytes(P2, lf, SC_THREADS, VT);
     PJ_CUDA(set_smem(kern, smem));
     const int grid = std::min(n_items, sm_count());
-    kern<<<grid, SC_THREADS, smem, st>>>(in, it, n_items, f, P2, bcap, off,
-                                        out, static_cast<uint32_t>(std::min<int64_t>(cap, UINT32_MAX)), status);
+    kern<<<grid, SC_THREADS, smem, st>>>(in, it, n_items, f, P2, lf, W, off, out,
+                                        static_cast<uint32_t>(std::min<int64_t>(cap, UINT32_MAX)), status);
     PJ_CUDA(cudaGetLastError());
     return PJ_OK;
 }
@@ -832,14 +887,7 @@ pj_status partition_pass2(const pj_plan* p, const Layout& L, int side, uint8_t* 
     if ((s = launch_scan(counts, static_cast<int64_t>(P2) * n_items, static_cast<uint32_t>(W2), off, tiles,
                                    ctr + (side == 0 ? CTR_BTILE2 : CTR_PTILE2), status, st)) != PJ_OK)
         return s;
-    switch (W2) {
-    case 2: return launch_scatter_tuples<K, 2>(in, it, n_items, f, P2, off, out, cap, status, st);
-    case 4: return launch_scatter_tuples<K, 4>(in, it, n_items, f, P2, off, out, cap, status, st);
-    case 8: return launch_scatter_tuples<K, 8>(in, it, n_items, f, P2, off, out, cap, status, st);
-    case 16: return launch_scatter_tuples<K, 16>(in, it, n_items, f, P2, off, out, cap, status, st);
-    case 32: return launch_scatter_tuples<K, 32>(in, it, n_items, f, P2, off, out, cap, status, st);
-    default: return PJ_ERR_INVALID;
-    }
+    return launch_scatter_tuples<K>(in, it, n_items, f, P2, W2, off, out, cap, status, st);
 }
 
 // Payload columns of the pairs written (no-op without them).
@@ -1015,7 +1063,8 @@ pj_status run_join(const pj_join_desc* d, const pj_plan* p, const Layout& L, uin
         return s;
     // the partitions the join reads: second-pass output for two-pass plans
     const size_t jb_off = two ? L.b_off2 : L.b_off, jp_off = two ? L.p_off2 : L.p_off;
-    const int jb_items = two ? L.C : L.b_items, jp_items = two ? L.C : L.p_items;
+    const int jb_items = two ? L.C : L.b_ipg, jp_items = two ? L.C : L.p_ipg;
+    const int jb_groups = two ? 1 : L.b_groups, jp_groups = two ? 1 : L.p_groups;
     E.mark(PJ_STAGE_JOIN_PLAN, st);
     if (hc.hs) {  // the heavy pairs [0, H) precede every join chunk
         heavy_total_kernel<<<1, 32, 0, st>>>(hc.out.item_count, L.p_items, heavy_total,
@@ -1028,7 +1077,7 @@ pj_status run_join(const pj_join_desc* d, const pj_plan* p, const Layout& L, uin
     const int position_chunk = std::max(16, cap_tuples / 16 * 16);
     join_items_kernel<<<(L.P + 255) / 256, 256, 0, st>>>(
         reinterpret_cast<int64_t*>(ws + jb_off), reinterpret_cast<int64_t*>(ws + jp_off), jb_items, jp_items,
-        L.P, reinterpret_cast<int32_t*>(ws + L.b_tot), reinterpret_cast<int32_t*>(ws + L.p_tot),
+        jb_groups, jp_groups, L.P, reinterpret_cast<int32_t*>(ws + L.b_tot), reinterpret_cast<int32_t*>(ws + L.p_tot),
         hash_split ? cap_tuples : position_chunk, p->probe_chunk, hash_split ? 1 : 0, MAX_SPLIT_LOG2,
         reinterpret_cast<int32_t*>(ws + L.split), reinterpret_cast<int64_t*>(ws + L.items), status, nullptr);
     PJ_CUDA(cudaGetLastError());
@@ -1047,6 +1096,8 @@ pj_status run_join(const pj_join_desc* d, const pj_plan* p, const Layout& L, uin
     a.probe_off = reinterpret_cast<const int64_t*>(ws + jp_off);
     a.b_items = jb_items;
     a.p_items = jp_items;
+    a.b_groups = jb_groups;
+    a.p_groups = jp_groups;
     a.P = L.P;
     // top hash bits the partition digits consumed
     a.digit_bits = (p->digit_mode == PJ_DIGIT_HASH ? p->bits1 : 0) + (two ? p->bits2 : 0);
@@ -1090,9 +1141,9 @@ pj_status resolve_plan(const pj_join_desc* d, const pj_plan* in, pj_plan* out)
     return check_plan(d, out);
 }
 
-pj_status check_ws(const pj_join_desc* d, const pj_plan* p, void* ws, size_t ws_bytes, Layout* L)
+pj_status check_ws(const pj_join_desc* d, const pj_plan* p, void* ws, size_t ws_bytes, Layout* L, bool grouped = true)
 {
-    *L = make_layout(d, p);
+    *L = make_layout(d, p, grouped);
     if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u) || ws_bytes < L->total) return PJ_ERR_WORKSPACE;
     return PJ_OK;
 }
@@ -1357,7 +1408,7 @@ pj_status pj_diag_scan_timeout(const pj_join_desc* d, const pj_plan* plan, void*
     Layout L;
     pj_status s = prepare(d, plan, ws, ws_bytes, &p, &L);
     if (s != PJ_OK) return s;
-    const int64_t m = static_cast<int64_t>(L.P1) * L.b_items;
+    const int64_t m = static_cast<int64_t>(L.P1) * L.b_items;  // (at most the counters there are)
     const int64_t ntiles = (m + SCAN_TILE - 1) / SCAN_TILE;
     if (withhold_tile < 0 || withhold_tile + 1 >= ntiles || spin_limit == 0) return PJ_ERR_INVALID;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1446,7 +1497,7 @@ pj_status pj_partitioned_capacity(int64_t n, int32_t key_bytes, const pj_plan* p
     d.n_build = n;
     d.key_bytes = key_bytes;
     d.unique_build_keys = 1;
-    const Layout L = make_layout(&d, plan);
+    const Layout L = make_layout(&d, plan, false);
     *tuples = plan->passes == 2 ? L.b_cap2 : L.b_cap;
     return PJ_OK;
 }
@@ -1467,7 +1518,7 @@ pj_status pj_partition(const void* keys, int64_t n, int32_t key_bytes, const pj_
     if (n > 0 && !aligned16(keys)) return PJ_ERR_ALIGNMENT;
     if (reinterpret_cast<uintptr_t>(tuples) & 15u) return PJ_ERR_ALIGNMENT;
     Layout L;
-    if ((s = check_ws(&d, plan, ws, ws_bytes, &L)) != PJ_OK) return s;
+    if ((s = check_ws(&d, plan, ws, ws_bytes, &L, false)) != PJ_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* w = static_cast<uint8_t*>(ws);
     PJ_CUDA(cudaMemsetAsync(w, 0, L.ctrl_end, st));
@@ -1775,24 +1826,14 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
                                    reinterpret_cast<uint64_t*>(w + lb.o_tiles), ctr + CTR_BTILE, status, st)) != PJ_OK)
         return s;
     constexpr int VT = sizeof(K) == 4 ? 4 : 2;
-    const size_t ssmem = scatter_smem(sizeof(K), lb.wc_cap, lb.Pmax);
+    const int lf = unit_logf<K>(lb.Pmax, lb.W, VT, 0);
+    if (lf < 0) return PJ_ERR_INVALID;
+    const size_t ssmem = WcUnits<K>::bytes(lb.Pmax, lf, SC_THREADS, VT);
     const uint32_t out_cap = static_cast<uint32_t>(std::min<int64_t>(lb.tuples, UINT32_MAX));
     const int sgrid = std::min(n_items, sm_count());
-    switch (lb.W) {
-    case 4: {
-        auto* k = scatter_seg_kernel<K, SC_THREADS, VT, 4>;
-        PJ_CUDA(set_smem(k, ssmem));
-        k<<<sgrid, SC_THREADS, ssmem, st>>>(items, n_items, lb.Pmax, lb.wc_cap, off, tuples, out_cap, status);
-        break;
-    }
-    case 2: {
-        auto* k = scatter_seg_kernel<K, SC_THREADS, VT, 2>;
-        PJ_CUDA(set_smem(k, ssmem));
-        k<<<sgrid, SC_THREADS, ssmem, st>>>(items, n_items, lb.Pmax, lb.wc_cap, off, tuples, out_cap, status);
-        break;
-    }
-    default: return PJ_ERR_INVALID;
-    }
+    auto* scatter = scatter_seg_kernel<K, SC_THREADS, VT>;
+    PJ_CUDA(set_smem(scatter, ssmem));
+    scatter<<<sgrid, SC_THREADS, ssmem, st>>>(items, n_items, lb.Pmax, lf, lb.W, off, tuples, out_cap, status);
     PJ_CUDA(cudaGetLastError());
     // work split over all partitions, then one join launch
     const PartRef* parts = reinterpret_cast<const PartRef*>(w + lb.o_parts);
@@ -1800,7 +1841,7 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
     const bool hash_split = lb.unique;
     const int position_chunk = std::max(16, cap_tuples / 16 * 16);
     join_items_kernel<<<(lb.G + 255) / 256, 256, 0, st>>>(
-        off, off, 1, 1, lb.G, totals, totals + lb.G, hash_split ? cap_tuples : position_chunk, lb.probe_chunk,
+        off, off, 1, 1, 1, 1, lb.G, totals, totals + lb.G, hash_split ? cap_tuples : position_chunk, lb.probe_chunk,
         hash_split ? 1 : 0, MAX_SPLIT_LOG2, reinterpret_cast<int32_t*>(w + lb.o_split),
         reinterpret_cast<int64_t*>(w + lb.o_jitems), status, parts);
     PJ_CUDA(cudaGetLastError());
@@ -1815,6 +1856,7 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
     a.build_tuples = a.probe_tuples = tuples;
     a.build_off = a.probe_off = off;
     a.b_items = a.p_items = 1;
+    a.b_groups = a.p_groups = 1;
     a.P = lb.G;
     a.split = reinterpret_cast<const int32_t*>(w + lb.o_split);
     a.item_off = reinterpret_cast<const int64_t*>(w + lb.o_item_off);
@@ -1838,8 +1880,8 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
         PJ_CUDA(cudaGetLastError());
         return PJ_OK;
     };
-    if (lb.unique) return launch(join_kernel<K, TABLE_BUCKET, true, true, false, JN_THREADS, true>);
-    return launch(join_kernel<K, TABLE_BUCKET, false, false, false, JN_THREADS, true>);
+    if (lb.unique) return launch(join_kernel<K, TABLE_BUCKET, true, true, false, JN_THREADS, 1, true>);
+    return launch(join_kernel<K, TABLE_BUCKET, false, false, false, JN_THREADS, 1, true>);
 }
 
 }  // namespace
@@ -1870,7 +1912,6 @@ pj_status large_batch_layout(const pj_join_desc* descs, const std::vector<int>& 
     for (const J& j : take) lb.Pmax = std::max(lb.Pmax, 1 << j.bits);
     lb.W = pick_wc(lb.key_bytes, ilog2_floor(lb.Pmax));
     if (lb.W == 0) return PJ_ERR_INVALID;
-    lb.wc_cap = wc_cap(lb.key_bytes, lb.W, lb.Pmax, SC_THREADS * (lb.key_bytes == 4 ? 4 : 2), 0);
     // probe chunks: about 8 work items per SM over the whole batch
     {
         const int64_t per = (probe_total + static_cast<int64_t>(sm_count()) * 8 - 1) / (static_cast<int64_t>(sm_count()) * 8);

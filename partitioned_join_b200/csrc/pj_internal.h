@@ -26,7 +26,7 @@ struct LargeBatch {
     bool unique = true;           // every join has unique build keys
     int G = 0;                    // partitions over all joins
     int64_t n_counts = 0;         // counters over all segments
-    int Pmax = 1, W = 4, wc_cap = 4;
+    int Pmax = 1, W = 4;
     int64_t tuples = 0;           // tuple buffer capacity (tuples)
     int64_t max_items = 0;        // join work items the buffers hold
     int table_cap = 0, nb_log2 = 0, probe_chunk = 0;

@@ -53,6 +53,7 @@ namespace pj {
 
 constexpr uint32_t EMPTY_ROW = 0xffffffffu;
 enum : int { TABLE_BUCKET = 0, TABLE_OPEN = 1, TABLE_COMPACT = 2, TABLE_EXACT = 3 };
+constexpr int MAX_GROUPS = 16;  // contiguous ranges a partition is made of
 constexpr int64_t COMPACT_RANGE = 65536;  // build range a COMPACT entry's index can address
 
 __global__ void zero_job_counts_kernel(const JobOut* __restrict__ outs, int32_t n)
@@ -63,10 +64,12 @@ __global__ void zero_job_counts_kernel(const JobOut* __restrict__ outs, int32_t 
 struct JoinArgs {
     const uint32_t* build_tuples;
     const uint32_t* probe_tuples;
-    const int64_t* build_off;   // partition p = [build_off[p*b_items], build_off[(p+1)*b_items])
-    const int64_t* probe_off;
-    int32_t b_items;
+    const int64_t* build_off;   // partition p = the ranges [build_off[(g*P+p)*b_items], build_off[(g*P+p+1)*b_items])
+    const int64_t* probe_off;   //   of the groups g, one after another
+    int32_t b_items;            // segments of a partition in a group
     int32_t p_items;
+    int32_t b_groups;           // at most MAX_GROUPS
+    int32_t p_groups;
     int32_t P;
     int32_t digit_bits;         // top hash bits consumed by partition digits (HASH digits), else 0
     const int32_t* split;       // per partition: log2 S_p (hash split) or S_p (position split)
@@ -99,7 +102,7 @@ struct JoinArgs {
 // Items per partition (S_p x K_p) and the split of partition p.
 // Batches pass `parts` (the partition's segments); single joins nullptr.
 __global__ void join_items_kernel(const int64_t* __restrict__ build_off, const int64_t* __restrict__ probe_off,
-                                  int32_t b_items, int32_t p_items, int32_t P,
+                                  int32_t b_items, int32_t p_items, int32_t b_groups, int32_t p_groups, int32_t P,
                                   const int32_t* __restrict__ build_tot, const int32_t* __restrict__ probe_tot,
                                   int32_t cap_per_table, int32_t probe_chunk, int32_t hash_split,
                                   int32_t max_split_log2, int32_t* __restrict__ split_out,
@@ -116,7 +119,9 @@ __global__ void join_items_kernel(const int64_t* __restrict__ build_off, const i
         p_items = parts[p].p_items;
     }
     const int64_t bc = build_tot[p], pc = probe_tot[p];
-    const int64_t prange = probe_off[p_at + p_items] - probe_off[p_at];
+    int64_t prange = 0;
+    for (int g = 0; g < p_groups; ++g, p_at += static_cast<int64_t>(P) * p_items)
+        prange += probe_off[p_at + p_items] - probe_off[p_at];
     int64_t items = 0;
     int32_t split = 0;
     if (bc > 0 && pc > 0) {
@@ -129,7 +134,9 @@ __global__ void join_items_kernel(const int64_t* __restrict__ build_off, const i
             split = lg;
             S = 1ll << lg;
         } else {
-            const int64_t brange = build_off[b_at + b_items] - build_off[b_at];
+            int64_t brange = 0;
+            for (int g = 0; g < b_groups; ++g, b_at += static_cast<int64_t>(P) * b_items)
+                brange += build_off[b_at + b_items] - build_off[b_at];
             S = (brange + cap_per_table - 1) / cap_per_table;
             if (S < 1) S = 1;
             split = static_cast<int32_t>(S);
@@ -423,21 +430,59 @@ constexpr int64_t PROBE_PREFETCH_BYTES = 128 << 10;
 
 // Output geometry.
 constexpr int OUT_CHUNK = 8192;  // entries a CTA claims per global atomic
-constexpr int OUT_SLOTS = 16;    // chunk bases a CTA keeps in shared memory
+constexpr int OUT_SLOTS = 8;     // chunk bases a CTA keeps in shared memory
 constexpr int JOIN_U = 4;        // probe tuples in flight per lane
 constexpr int JOIN_BU = 4;       // build tuples in flight per thread
 
-// Where one work item's tuples are.  Thread 0 works it out for the next
-// item while the current one probes, so an item starts without a chain of
-// dependent global loads (item -> partition -> offsets).
+constexpr uint32_t JOIN_STEP = 128;  // tuples a warp takes at a time (32 lanes x JOIN_U = JOIN_BU)
+static_assert(JOIN_U * 32 == JOIN_STEP && JOIN_BU * 32 == JOIN_STEP, "a step is U tuples a lane");
+
+// One work item.  Warp 0 works out the next one while the current one probes,
+// so an item starts without a chain of dependent global loads (item ->
+// partition -> offsets).
 struct ItemMeta {
-    int64_t b_lo, b_hi;  // build tuples of the item's piece
-    int64_t q_lo, q_hi;  // probe tuples of the item's chunk
-    int32_t p;           // partition
-    int32_t piece;       // build piece (hash split: the piece's hash bits)
-    int32_t sbits;       // hash split bits (0: no hash split)
-    int32_t dbits;       // top hash bits the partition digits consumed
-    JobOut jout;         // batches: the item's join
+    int32_t p;      // partition
+    int32_t piece;  // build piece (hash split: the piece's hash bits)
+    int32_t sbits;  // hash split bits (0: no hash split)
+    int32_t dbits;  // top hash bits the partition digits consumed
+};
+
+// One side's tuples of an item as steps of at most JOIN_STEP tuples, none
+// across two of the partition's ranges: range g's steps are [last[g - 1],
+// last[g]) and cover n[g] tuples from tuple start[g] on.  A warp looks its
+// range up with one ballot.  (Walking all ranges by position, each lane with
+// its own place, broke up the unrolled loads: 2^27 x 2^27 int32 join 0.98 ->
+// 1.28 ms.)
+template <int NG>
+struct ItemSteps {
+    uint32_t last[NG];
+    uint32_t start[NG];
+    uint32_t n[NG];
+};
+
+// A warp's place in one side: the range it is in.  Its steps only grow within
+// a pass, so it moves on a few times per item, and a step costs a warp-uniform
+// compare.  at(): this lane's first tuple of step st; left: tuples from it on,
+// so its u-th load is 32 u tuples further and exists while 32 u < left --
+// immediates both, where an index for every load took 9 more instructions per
+// 32 tuples.  The range's numbers stay in shared memory (a read per step):
+// kept in registers they made the probe spill.
+template <int NG, int WORDS>
+struct StepCursor {
+    int g = 0;
+    __device__ __forceinline__ const uint32_t* at(const ItemSteps<NG>& r, const uint32_t* tuples, uint32_t st, int& left)
+    {
+        const uint32_t lane = threadIdx.x & 31;
+        uint32_t first = 0;
+        if constexpr (NG > 1) {
+            if (st >= r.last[g])
+                g = __popc(__ballot_sync(0xffffffffu, lane < NG && st >= r.last[lane < NG ? lane : 0]));
+            first = g > 0 ? r.last[g - 1] : 0u;
+        }
+        const uint32_t i = (st - first) * JOIN_STEP + lane;
+        left = static_cast<int>(r.n[g] - i);
+        return tuples + static_cast<size_t>(r.start[g] + i) * WORDS;
+    }
 };
 
 template <typename K, int TABLE>
@@ -462,7 +507,7 @@ struct JoinSmem {
     __host__ __device__ static size_t bytes(int cap, int nb_log2) { return table_bytes(cap, nb_log2); }
 };
 
-template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF, int THREADS, bool BATCH = false>
+template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF, int THREADS, int NG, bool BATCH = false>
 __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
 {
     using TV = TupleView<K>;
@@ -487,7 +532,11 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
     __shared__ uint32_t s_warp[NWARPS];
     __shared__ int s_nbuild;
     __shared__ uint32_t s_step;  // next probe step of the current item
-    __shared__ ItemMeta s_cur, s_nxt;  // the current and the next item
+    // the current and the next item, their build and probe tuples (copied over
+    // at an item's start: fixed addresses cost the loops no registers)
+    __shared__ ItemMeta s_meta, s_nmeta;
+    __shared__ ItemSteps<NG> s_bst, s_qst, s_nbst, s_nqst;
+    __shared__ JobOut s_jout, s_njout;
 
     const uint64_t stream_pol = l2_evict_first_policy();
     const int NB = 1 << a.nb_log2;
@@ -495,8 +544,10 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
     const int64_t total_items = a.item_off[a.P];
     const bool write_out = a.out_build != nullptr;
 
-    auto load_meta = [&](int64_t it) -> ItemMeta {
-        ItemMeta m;
+    // Warp 0: item `it` as the next item.  prev_p: the build tuples are fetched
+    // into L2 unless that partition's are there already (COMPACT tables: see
+    // the call).
+    auto load_meta = [&](int64_t it, int prev_p) {
         const int p = a.item_part[it];
         const int64_t local = it - a.item_off[p];
         const int32_t split = a.split[p];
@@ -505,39 +556,74 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
         const int64_t pchunk = local / S;
         int64_t b_at = static_cast<int64_t>(p) * a.b_items, p_at = static_cast<int64_t>(p) * a.p_items;
         int32_t b_n = a.b_items, p_n = a.p_items;
-        m.dbits = a.digit_bits;
-        m.jout = JobOut{};
         if constexpr (BATCH) {
-            const PartRef r = a.parts[p];
+            const PartRef& r = a.parts[p];
             b_at = r.b_at;
             p_at = r.p_at;
             b_n = r.b_items;
             p_n = r.p_items;
-            m.dbits = r.digit_bits;
-            m.jout = a.outs[r.job];
         }
-        const int64_t b_lo0 = a.build_off[b_at];
-        const int64_t b_hi0 = a.build_off[b_at + b_n];
-        m.b_lo = b_lo0;
-        m.b_hi = b_hi0;
-        if (!HASH_SPLIT) {
-            m.b_lo = b_lo0 + piece * a.position_chunk;
-            m.b_hi = m.b_lo + a.position_chunk < b_hi0 ? m.b_lo + a.position_chunk : b_hi0;
-            if (m.b_lo > m.b_hi) m.b_lo = m.b_hi;
+        // positions [lo, hi) of one side's ranges, lane g taking range g
+        auto side = [&](const int64_t* off, int64_t at, int32_t segs, int64_t stride, int groups, int64_t lo, int64_t hi,
+                        ItemSteps<NG>& out, uint32_t& start, uint32_t& n) {
+            int64_t s = 0, len = 0;
+            if (lane < groups) {
+                s = off[at + lane * stride];
+                len = off[at + lane * stride + segs] - s;
+            }
+            int64_t end = len;
+#pragma unroll
+            for (int o = 1; o < NG; o <<= 1) {
+                const int64_t x = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= o) end += x;
+            }
+            const int64_t from = lo > end - len ? lo : end - len, to_ = hi < end ? hi : end;
+            n = to_ > from ? static_cast<uint32_t>(to_ - from) : 0u;
+            start = static_cast<uint32_t>(s + (from - (end - len)));
+            uint32_t last = (n + JOIN_STEP - 1) / JOIN_STEP;
+#pragma unroll
+            for (int o = 1; o < NG; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, last, o);
+                if (lane >= o) last += x;
+            }
+            if (lane < NG) {
+                out.last[lane] = last;
+                out.start[lane] = start;
+                out.n[lane] = n;
+            }
+        };
+        const int64_t all = int64_t(1) << 40;
+        uint32_t start, n;
+        side(a.probe_off, p_at, p_n, static_cast<int64_t>(a.P) * a.p_items, a.p_groups, pchunk * a.probe_chunk,
+             (pchunk + 1) * a.probe_chunk, s_nqst, start, n);
+        side(a.build_off, b_at, b_n, static_cast<int64_t>(a.P) * a.b_items, a.b_groups,
+             HASH_SPLIT ? 0 : piece * a.position_chunk, HASH_SPLIT ? all : (piece + 1) * a.position_chunk, s_nbst, start, n);
+        if (TABLE != TABLE_COMPACT && p != prev_p && n > 0) {
+            const int64_t nbytes = static_cast<int64_t>(n) * TV::WORDS * 4;
+            prefetch_l2(a.build_tuples + static_cast<int64_t>(start) * TV::WORDS, nbytes < (1 << 20) ? nbytes : (1 << 20));
         }
-        const int64_t q_lo0 = a.probe_off[p_at];
-        const int64_t q_hi0 = a.probe_off[p_at + p_n];
-        m.q_lo = q_lo0 + pchunk * a.probe_chunk;
-        m.q_hi = m.q_lo + a.probe_chunk < q_hi0 ? m.q_lo + a.probe_chunk : q_hi0;
-        m.p = p;
-        m.piece = static_cast<int32_t>(piece);
-        m.sbits = HASH_SPLIT ? split : 0;
-        return m;
+        if (lane == 0) {
+            ItemMeta m;
+            m.p = p;
+            m.piece = static_cast<int32_t>(piece);
+            m.sbits = HASH_SPLIT ? split : 0;
+            m.dbits = a.digit_bits;
+            if constexpr (BATCH) {
+                const PartRef& r = a.parts[p];
+                m.dbits = r.digit_bits;
+                s_njout = a.outs[r.job];
+            }
+            s_nmeta = m;
+        }
     };
-    if (threadIdx.x == 0) {
-        s_q = 0;
-        s_next = static_cast<int64_t>(atomicAdd(a.queue, 1u));
-        if (s_next < total_items && s_next < a.max_items) s_nxt = load_meta(s_next);
+    if (threadIdx.x < 32) {
+        int64_t it = 0;
+        if (lane == 0) {
+            s_q = 0;
+            s_next = it = static_cast<int64_t>(atomicAdd(a.queue, 1u));
+        }
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it < total_items && it < a.max_items) load_meta(it, -1);
     }
     if (threadIdx.x < OUT_SLOTS) s_cslot[threadIdx.x] = ~0ull;
 
@@ -665,44 +751,48 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                 }
         }
     };
-    bool first_item = true;
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) {
-            s_item = s_next;
-            s_cur = s_nxt;
-            s_next = static_cast<int64_t>(atomicAdd(a.queue, 1u));  // claim the next item early
+        if (threadIdx.x < 32) {
+            if (lane == 0) {
+                s_item = s_next;
+                s_meta = s_nmeta;
+                if constexpr (BATCH) s_jout = s_njout;
+                s_next = static_cast<int64_t>(atomicAdd(a.queue, 1u));  // claim the next item early
+            }
+            if (lane < NG) {
+                s_bst.last[lane] = s_nbst.last[lane];
+                s_bst.start[lane] = s_nbst.start[lane];
+                s_bst.n[lane] = s_nbst.n[lane];
+                s_qst.last[lane] = s_nqst.last[lane];
+                s_qst.start[lane] = s_nqst.start[lane];
+                s_qst.n[lane] = s_nqst.n[lane];
+            }
         }
         __syncthreads();
         const int64_t item = s_item;
         if (item >= total_items || item >= a.max_items) break;
-        const int p = s_cur.p;
-        const int64_t piece = s_cur.piece;
-        const int sbits = s_cur.sbits;
-        const int dbits = s_cur.dbits;
-        const int64_t b_lo = s_cur.b_lo, b_hi = s_cur.b_hi;
-        const int64_t q_lo = s_cur.q_lo, q_hi = s_cur.q_hi;
-        if constexpr (BATCH) jout = s_cur.jout;
+        const int p = s_meta.p;
+        const uint32_t piece = static_cast<uint32_t>(s_meta.piece);
+        const int sbits = s_meta.sbits;
+        const int dbits = s_meta.dbits;
+        if constexpr (BATCH) jout = s_jout;
         const int skip = dbits + sbits;
         const int piece_shift = 32 - (sbits > 0 ? sbits : 1);
 
-        // a CTA's first item: its build range was not prefetched during an
-        // earlier probe phase
-        if (TABLE != TABLE_COMPACT && first_item && threadIdx.x == 0 && b_hi > b_lo) {
-            const int64_t bbytes = (b_hi - b_lo) * TV::WORDS * 4;
-            prefetch_l2(a.build_tuples + b_lo * TV::WORDS, bbytes < (1 << 20) ? bbytes : (1 << 20));
-        }
-        first_item = false;
         // the head of the probe chunk streams into L2 while the table is built
-        if (threadIdx.x == 0) {
-            const int64_t pbytes = (q_hi - q_lo) * TV::WORDS * 4;
-            prefetch_l2_stream(a.probe_tuples + (q_lo * TV::WORDS),
-                               pbytes < PROBE_PREFETCH_BYTES ? pbytes : PROBE_PREFETCH_BYTES, stream_pol);
+        if (threadIdx.x < NG) {
+            const int64_t head = PROBE_PREFETCH_BYTES / (TV::WORDS * 4);
+            const int64_t left = head - (lane > 0 ? static_cast<int64_t>(s_qst.last[lane - 1]) * JOIN_STEP : 0);
+            const int64_t n = s_qst.n[lane] < left ? s_qst.n[lane] : left;
+            if (n > 0)
+                prefetch_l2_stream(a.probe_tuples + static_cast<int64_t>(s_qst.start[lane]) * TV::WORDS,
+                                   n * TV::WORDS * 4, stream_pol);
         }
 
         auto in_piece = [&](uint32_t h) -> bool {
             if (!HASH_SPLIT || sbits == 0) return true;
-            return static_cast<int64_t>((h << dbits) >> piece_shift) == piece;
+            return ((h << dbits) >> piece_shift) == piece;
         };
         auto bucket_of = [&](uint32_t h) -> uint32_t { return h & nb_mask; };
         auto finger_of = [&](uint32_t h) -> uint32_t { return (h >> a.nb_log2) & 0xffffu; };
@@ -714,11 +804,14 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
             return SLOT_REF ? slot_ref(h, a.cap) : slot_fast(h, skip, static_cast<uint32_t>(a.cap));
         };
 
+        // COMPACT: the build range is one contiguous range (one group)
+        const int64_t build0 = s_bst.start[0];
+        const uint32_t b_total = s_bst.last[NG - 1], warp = threadIdx.x >> 5;
         if (threadIdx.x == 0) s_step = 0;  // ordered before the probe by the build's barriers
 
         // ---- build ----
         bool skip_item = false;
-        if (TABLE == TABLE_COMPACT && b_hi - b_lo > COMPACT_RANGE) {
+        if (TABLE == TABLE_COMPACT && s_bst.n[0] > COMPACT_RANGE) {
             // an entry's 16-bit index cannot address this range: the planner avoids it
             if (threadIdx.x == 0) raise_status(a.status, ST_OVERFLOW);
             skip_item = true;
@@ -737,20 +830,18 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                 uint32_t nh[JOIN_BU];
                 Cmp nk[JOIN_BU];
                 int32_t nr[JOIN_BU];
-                // 32-bit offsets in the item's build range
-                const uint32_t* bt = a.build_tuples + b_lo * TV::WORDS;
-                const uint32_t bn = static_cast<uint32_t>(b_hi - b_lo);
-                auto load_batch = [&](uint32_t i0) {
+                StepCursor<NG, TV::WORDS> cur;
+                auto load_step = [&](uint32_t st) {
+                    int left;
+                    const uint32_t* t = cur.at(s_bst, a.build_tuples, st, left);
 #pragma unroll
                     for (int u = 0; u < JOIN_BU; ++u) {
-                        const uint32_t i = i0 + u * THREADS;
                         nr[u] = -1;
-                        if (i < bn) TV::load(bt, i, nh[u], nk[u], nr[u]);
+                        if (u * 32 < left) TV::load(t, u * 32, nh[u], nk[u], nr[u]);
                     }
                 };
-                uint32_t i0 = threadIdx.x;
-                if (i0 < bn) load_batch(i0);
-                for (; i0 < bn; i0 += THREADS * JOIN_BU) {
+                if (warp < b_total) load_step(warp);
+                for (uint32_t st = warp; st < b_total; st += NWARPS) {
                     uint32_t h[JOIN_BU];
                     int32_t r[JOIN_BU];
 #pragma unroll
@@ -758,7 +849,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                         h[u] = nh[u];
                         r[u] = nr[u];
                     }
-                    if (i0 + THREADS * JOIN_BU < bn) load_batch(i0 + THREADS * JOIN_BU);
+                    if (st + NWARPS < b_total) load_step(st + NWARPS);
 #pragma unroll
                     for (int u = 0; u < JOIN_BU; ++u) {
                         if (r[u] >= 0 && in_piece(h[u])) {
@@ -778,17 +869,17 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
             } else {
                 scan_u16_pairs<THREADS>(ends, NB / 2 + 1, s_warp);
                 // pass 2: place
-                const uint32_t* bt = a.build_tuples + b_lo * TV::WORDS;
-                const uint32_t bn = static_cast<uint32_t>(b_hi - b_lo);
-                for (uint32_t i0 = threadIdx.x; i0 < bn; i0 += THREADS * JOIN_BU) {
+                StepCursor<NG, TV::WORDS> cur;
+                for (uint32_t st = warp; st < b_total; st += NWARPS) {
+                    int left;
+                    const uint32_t* t = cur.at(s_bst, a.build_tuples, st, left);
                     uint32_t h[JOIN_BU];
                     Cmp k[JOIN_BU];
                     int32_t r[JOIN_BU];
 #pragma unroll
                     for (int u = 0; u < JOIN_BU; ++u) {
-                        const uint32_t i = i0 + u * THREADS;
                         r[u] = -1;
-                        if (i < bn) TV::load(bt, i, h[u], k[u], r[u]);
+                        if (u * 32 < left) TV::load(t, u * 32, h[u], k[u], r[u]);
                     }
 #pragma unroll
                     for (int u = 0; u < JOIN_BU; ++u) {
@@ -797,7 +888,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                             const uint32_t old = atomicAdd(&ends[b >> 1], (b & 1u) ? 0x10000u : 1u);
                             const int pos = static_cast<int>((b & 1u) ? (old >> 16) : (old & 0xffffu));
                             if constexpr (TABLE == TABLE_COMPACT)
-                                ctab[pos] = (finger_of(h[u]) << 16) | (i0 + u * THREADS);
+                                ctab[pos] = (finger_of(h[u]) << 16) | (st * JOIN_STEP + u * 32 + lane);
                             else if constexpr (TABLE == TABLE_EXACT)
                                 ExactEntry<K>::put(table, pos, (xfinger_of(h[u]) << a.row_bits) | static_cast<uint32_t>(r[u]),
                                                    ExactEntry<K>::key_lo(k[u]));
@@ -814,11 +905,16 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                 else orows[i] = EMPTY_ROW;
             }
             __syncthreads();
-            for (int64_t i = b_lo + threadIdx.x; i < b_hi; i += THREADS) {
-                uint32_t h;
+            StepCursor<NG, TV::WORDS> cur;
+            for (uint32_t s4 = warp; s4 < b_total * JOIN_BU; s4 += NWARPS) {
+                uint32_t h = 0;
                 Cmp k;
-                int32_t r;
-                TV::load(a.build_tuples, i, h, k, r);
+                int32_t r = -1;
+                __syncwarp();
+                int left;
+                const uint32_t* t = cur.at(s_bst, a.build_tuples, s4 / JOIN_BU, left);
+                const int i = (s4 % JOIN_BU) * 32;
+                if (i < left) TV::load(t, i, h, k, r);
                 if (r < 0 || !in_piece(h)) continue;
                 uint32_t sl = slot_of(h);
                 int tries = 0;
@@ -845,34 +941,32 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
         // for COMPACT tables: their fingerprint checks re-read build tuples
         // and the prefetched ranges were evicted before use (0.83 GB more
         // DRAM reads at 2^27 x 2^27, no time gained).
-        if (threadIdx.x == 0 && s_next < total_items && s_next < a.max_items) {
-            s_nxt = load_meta(s_next);
-            if (TABLE != TABLE_COMPACT && s_nxt.p != p && s_nxt.b_hi > s_nxt.b_lo) {
-                const int64_t nbytes = (s_nxt.b_hi - s_nxt.b_lo) * TV::WORDS * 4;
-                prefetch_l2(a.build_tuples + s_nxt.b_lo * TV::WORDS, nbytes < (1 << 20) ? nbytes : (1 << 20));
-            }
+        if (threadIdx.x < 32) {
+            const int64_t next = s_next;
+            if (next < total_items && next < a.max_items) load_meta(next, p);
+            __syncwarp();
         }
 
         // ---- probe: warps run independently; loads run one step ahead ----
         if (!skip_item) {
             // warps claim steps of 32*U tuples from a shared counter, so they
             // finish the item together; the next claim's loads run ahead
-            const uint32_t* pbase = a.probe_tuples + q_lo * TV::WORDS;
-            const uint32_t qn = static_cast<uint32_t>(q_hi - q_lo);
-            constexpr uint32_t STEP = 32 * U;
+            const uint32_t qn = s_qst.last[NG - 1];
             uint32_t nh[U];
             Cmp nk[U];
             int32_t nr[U];
             auto claim = [&]() -> uint32_t {
                 uint32_t st = 0;
                 if (lane == 0) st = atomicAdd(&s_step, 1u);
-                return __shfl_sync(0xffffffffu, st, 0) * STEP;
+                return __shfl_sync(0xffffffffu, st, 0);
             };
-            auto load_step = [&](uint32_t s0) {
+            StepCursor<NG, TV::WORDS> cur;
+            auto load_step = [&](uint32_t st) {
+                int left;
+                const uint32_t* t = cur.at(s_qst, a.probe_tuples, st, left);
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const uint32_t i = s0 + u * 32 + lane;
-                    TV::load_stream_if(pbase, i, i < qn, nh[u], nk[u], nr[u], stream_pol);
+                    TV::load_stream_if(t, u * 32, u * 32 < left, nh[u], nk[u], nr[u], stream_pol);
                 }
             };
             uint32_t s0 = claim();
@@ -901,7 +995,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                             if ((e >> 16) == fq) {  // fingerprint hit: compare the full key
                                 Cmp bk;
                                 int32_t br;
-                                TV::load_key_row(a.build_tuples, b_lo + (e & 0xffffu), bk, br);
+                                TV::load_key_row(a.build_tuples, build0 + (e & 0xffffu), bk, br);
                                 if (bk == k[u]) {
                                     found = true;
                                     brow_u = static_cast<uint32_t>(br);
@@ -1020,7 +1114,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                             if (hit[u]) {
                                 Cmp bk;
                                 int32_t br;
-                                TV::load_key_row(a.build_tuples, b_lo + (ctab[at[u]] & 0xffffu), bk, br);
+                                TV::load_key_row(a.build_tuples, build0 + (ctab[at[u]] & 0xffffu), bk, br);
                                 if (bk == k[u]) {
                                     emit[u] = true;
                                     brow[u] = static_cast<uint32_t>(br);
@@ -1030,6 +1124,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                                 }
                             }
                         }
+                        __syncwarp();  // (the lanes' walks end apart)
                         if (!__any_sync(0xffffffffu, again)) break;
                     }
                     append_direct(emit, brow, r);
@@ -1169,6 +1264,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                             emit[u] = lookup(u, at_u, end_u, sl_u, steps_u, live_u, brow[u]);
                         }
                     }
+                    __syncwarp();
                     append_direct(emit, brow, r);
                 } else {
                     // repeated build keys: every tuple walks on, one match per lane per append
@@ -1190,6 +1286,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                             emit[u] = live[u] && lookup(u, at[u], end[u], sl[u], steps[u], live[u], brow[u]);
                             any_live |= live[u];
                         }
+                        __syncwarp();
                         append_direct(emit, brow, r);
                         if (!__any_sync(0xffffffffu, any_live)) break;
                     }

@@ -2,13 +2,17 @@
 // write-combining scatter.
 //
 // Layout of one partitioned column.  The input is cut into n_items equal
-// chunks ("items", one per resident scatter CTA).  Item i's tuples of
-// partition p form the segment [off[p*n_items + i], off[p*n_items + i + 1])
-// of the output, where off is the exclusive scan of the per-(p, i) counts,
-// each rounded up to W tuples.  So partitions are contiguous
-// (partition p = [off[p*n_items], off[(p+1)*n_items]) ), every segment starts
-// on a W-tuple boundary, and the padding tuples that fill a segment's last
-// W-group carry row = -1.
+// chunks ("items", one per resident scatter CTA), and the items into groups of
+// ipg.  Item i = (g, j) has one counter per partition at (g * P + p) * ipg + j;
+// off is the exclusive scan of these counts, each rounded up to W tuples, and
+// the item's tuples of partition p form the segment of that index.  So
+// partition p is one contiguous range per group,
+// [off[(g * P + p) * ipg], off[(g * P + p + 1) * ipg]), every segment starts on
+// a W-tuple boundary, and the padding tuples of a segment carry row = -1.
+// One group (ipg = n_items) makes partitions contiguous.  Large columns take
+// several: a scatter CTA then writes within its group's part of the buffer,
+// a few hundred MB that its address translation covers -- spread over all
+// 4.3 GB, plain sector stores took 2.5 ms instead of 1.8.
 //
 // Tuples.  4-byte keys are stored as {murmur(key), row}: MurmurHash3_x86_32
 // of a 4-byte key is a bijection of 32-bit values (every step -- odd
@@ -36,6 +40,13 @@
 #include "pj_types.cuh"
 
 namespace pj {
+
+// Index of item `item`'s first counter (partition 0) with the items in groups
+// of ipg: partition p's is p * ipg further.
+__device__ __forceinline__ int64_t seg_base(int item, int ipg, int P)
+{
+    return static_cast<int64_t>(item / ipg) * P * ipg + item % ipg;
+}
 
 template <typename K>
 __device__ __forceinline__ uint32_t key_digit(const DigitFn& f, K key)
@@ -88,7 +99,7 @@ constexpr int HIST_UNROLL = 4;  // 16-byte vectors in flight per thread
 template <typename K, bool HASHD, bool HEAVY>
 __global__ void __launch_bounds__(HIST_THREADS) hist_keys_kernel(const K* __restrict__ keys, int64_t n,
                                                                  int64_t chunk, int32_t n_items, int32_t hsplit,
-                                                                 DigitFn f, int32_t P,
+                                                                 DigitFn f, int32_t P, int32_t ipg,
                                                                  uint32_t* __restrict__ counts_T,
                                                                  int32_t* __restrict__ totals,
                                                                  typename HeavyArg<HEAVY>::type hs, HeavyOut ho)
@@ -161,7 +172,7 @@ __global__ void __launch_bounds__(HIST_THREADS) hist_keys_kernel(const K* __rest
     for (int p = threadIdx.x; p < P; p += HIST_THREADS) {
         const uint32_t c = cnt[p];
         if (c) {
-            atomicAdd(&counts_T[static_cast<int64_t>(p) * n_items + item], c);
+            atomicAdd(&counts_T[seg_base(item, ipg, P) + static_cast<int64_t>(p) * ipg], c);
             if (totals != nullptr) atomicAdd(&totals[p], static_cast<int32_t>(c));
         }
     }
@@ -369,6 +380,14 @@ __device__ __forceinline__ void st_global_v8(uint32_t* g, const uint4& a, const 
                  : "memory");
 }
 
+// The same with an L2 policy.
+__device__ __forceinline__ void st_global_v8_keep(uint32_t* g, const uint4& a, const uint4& b, uint64_t pol)
+{
+    asm volatile("st.global.L2::cache_hint.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8}, %9;" ::"l"(g), "r"(a.x),
+                 "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w), "l"(pol)
+                 : "memory");
+}
+
 template <typename K, int W>
 __device__ __forceinline__ void wc_flush(const uint32_t* sbuf, uint32_t* gdst)
 {
@@ -506,12 +525,458 @@ __device__ __forceinline__ void wc_finish(int P, uint32_t* buf, int cap, WcState
     }
 }
 
+// ---------------------------------------------------------------------------
+// Write-combining placement without block barriers.
+//
+// Per partition the CTA keeps one unit of F tuples (a power of two, about
+// 128 KB over all partitions) in shared memory, a fill word {parity, count},
+// a front cursor and a back cursor into the partition's segment.  A tuple
+// takes count c by a shared atomic on the fill word:
+//   c < F      it goes to slot c, its row's top bit set to the unit's parity
+//              (rows are below 2^31);
+//   c >= F     the unit is full and not yet written: the tuple goes straight
+//              to the back of the segment (back cursor, one atomic), so no
+//              thread ever waits for a unit and the front stays aligned;
+//   c == F - 1 the tuple's warp writes the unit: it notes {partition, parity}
+//              in the warp's list, and after its round the warp writes the
+//              listed units together, one 32-byte sector a lane.
+// A lane that writes a sector re-reads it until every row shows the unit's
+// parity: the other tuples of the unit took their slots before this one,
+// and nothing stands between a taken slot and its store, so the wait is a few
+// shared-memory latencies (bounded all the same).  Taking the sector into
+// registers frees the unit: the fill word moves to the other parity and
+// count 0 before the sector leaves.
+//
+// The block-wide form (three barriers per round of one vector a thread)
+// waited on shared-memory latency and barriers with half the issue slots
+// idle.  A count needs no reset bound: it grows by one per tuple of the
+// chunk at most, and a chunk has fewer than 2^24 tuples.
+constexpr int WCU_LATE = 64;  // tuples a warp keeps to place later
+constexpr uint32_t WCU_COUNT = (1u << 24) - 1u;  // count bits of a fill word; bit 24: parity
+
+template <typename K>
+struct WcUnits {
+    static constexpr int TW = TupleTraits<K>::WORDS;
+    static constexpr int CH = 8 / TW;  // tuples of a sector
+    static constexpr int LOG_CH = CH == 4 ? 2 : 1;
+    static constexpr int MAX_LOGF = LOG_CH + 5;  // a unit's sectors are written by one pass of a warp
+    uint32_t* buf;
+    uint32_t* fill;
+    uint32_t* cur;
+    uint32_t* back;
+    uint16_t* list;  // this warp's: one entry per tuple of a round
+    uint32_t* late;  // this warp's tuples that met a full unit (WCU_LATE)
+    uint16_t* late_d;  // and their partitions
+    int logF;
+    uint64_t keep, done;  // L2 policies of sectors that leave their line open / complete it (0: none)
+
+    // shared memory of P partitions, threads * v tuples a round
+    __host__ __device__ static size_t bytes(int P, int logF, int threads, int v)
+    {
+        return (static_cast<size_t>(P) << logF) * TW * 4 + static_cast<size_t>(threads / 32) * WCU_LATE * (TW * 4 + 2) +
+               static_cast<size_t>(P) * 12 + static_cast<size_t>(threads) * v * 2;
+    }
+    __device__ void bind(uint8_t* smem, int P, int lf, int v)
+    {
+        const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+        logF = lf;
+        buf = reinterpret_cast<uint32_t*>(smem);
+        // Many partitions: a line waits for its other sectors while the CTAs
+        // fill P x 148 others, and is written to HBM in parts if it is evicted
+        // meanwhile.  So its sectors are marked evict-last, the one that
+        // completes it evict-first: 4096 partitions of 2^27 int32 keys 0.81 ->
+        // 0.60 ms, of 2^28 int64 keys 2.94 -> 2.39 ms, 2048 of 2^26 int64 keys
+        // 0.49 -> 0.43 ms (without the demotion 0.605, 2.45, 0.43).  At 2048
+        // partitions of int32 keys, whose scatter waits on the SMs, the
+        // policy operands cost 4 %.
+        keep = done = 0;
+        if (P >= (CH == 4 ? 4096 : 2048)) {
+            asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
+            asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(done));
+        }
+        uint32_t* after = buf + (static_cast<size_t>(P) << lf) * TW;
+        late = after + warp * WCU_LATE * TW;
+        fill = after + warps * WCU_LATE * TW;
+        cur = fill + P;
+        back = cur + P;
+        uint16_t* half = reinterpret_cast<uint16_t*>(back + P);
+        late_d = half + warp * WCU_LATE;
+        list = half + warps * WCU_LATE + warp * 32 * v;
+    }
+};
+
+__device__ __forceinline__ uint4 lds_v4(const uint32_t* p)
+{
+    uint4 v;
+    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p)))
+                 : "memory");
+    return v;
+}
+
+template <int TW>
+__device__ __forceinline__ void sts_tuple(uint32_t* p, const uint32_t (&w)[TW], uint32_t row)
+{
+    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+    if constexpr (TW == 2)
+        asm volatile("st.volatile.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(w[0]), "r"(row) : "memory");
+    else
+        asm volatile("st.volatile.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(row)
+                     : "memory");
+}
+
+// Start of an item: empty units of parity 1 over slots of parity 0, cursors
+// at the ends of the item's segments.  off(p) / off_end(p): the segment.
+template <typename K, typename Off, typename OffEnd>
+__device__ __forceinline__ void wcu_begin(const WcUnits<K>& u, int P, Off off, OffEnd off_end)
+{
+    const int words4 = static_cast<int>((static_cast<size_t>(P) << u.logF) * WcUnits<K>::TW / 4);
+    for (int i = threadIdx.x; i < words4; i += blockDim.x) reinterpret_cast<uint4*>(u.buf)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int p = threadIdx.x; p < P; p += blockDim.x) {
+        u.fill[p] = 1u << 24;
+        u.cur[p] = static_cast<uint32_t>(off(p));
+        u.back[p] = static_cast<uint32_t>(off_end(p));
+    }
+    __syncthreads();
+}
+
+// Places a warp's tuples: w[v] = words, dv[v] = partition, ok[v] = real.
+// KEEP: tuples that meet a full unit go to the warp's late list (n_late of
+// them so far) while it has room.
+template <typename K, int V, bool KEEP>
+__device__ __forceinline__ void wcu_put(const WcUnits<K>& u, uint32_t& n_late,
+                                        const uint32_t (&w)[V][TupleTraits<K>::WORDS],
+                                        const uint32_t (&dv)[V], const bool (&ok)[V], uint32_t* __restrict__ out,
+                                        uint32_t out_cap, uint32_t* __restrict__ status)
+{
+    using U = WcUnits<K>;
+    constexpr int TW = U::TW;
+    const uint32_t F = 1u << u.logF;
+    const int lane = threadIdx.x & 31;
+    uint32_t old[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) old[v] = ok[v] ? atomicAdd(&u.fill[dv[v]], 1u) : WCU_COUNT;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const uint32_t c = old[v] & WCU_COUNT;
+        if (c < F)
+            sts_tuple<TW>(u.buf + (static_cast<size_t>(dv[v]) << u.logF) * TW + c * TW, w[v],
+                          w[v][TW - 1] | ((old[v] << 7) & 0x80000000u));
+    }
+    uint32_t n = 0;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const bool last = (old[v] & WCU_COUNT) == F - 1u;
+        const uint32_t bal = __ballot_sync(0xffffffffu, last);
+        if (last)
+            u.list[n + __popc(bal & ((1u << lane) - 1u))] = static_cast<uint16_t>(dv[v] | ((old[v] >> 9) & 0x8000u));
+        n += __popc(bal);
+    }
+    __syncwarp();
+    const int log_c = u.logF - U::LOG_CH;  // sectors of a unit
+    const uint32_t total = n << log_c;
+    for (uint32_t i0 = 0; i0 < total; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        const bool act = i < total;
+        const uint32_t e = act ? u.list[i >> log_c] : 0u;
+        const uint32_t p = e & 0x7fffu, c = i & ((1u << log_c) - 1u);
+        const uint32_t parity = (e >> 15) << 31;
+        const uint32_t* src = u.buf + (static_cast<size_t>(p) << u.logF) * TW + c * 8;
+        uint4 a, b;
+        uint32_t spins = 0;
+        for (;;) {
+            a = lds_v4(src);
+            b = lds_v4(src + 4);
+            uint32_t differ;
+            if constexpr (TW == 2)
+                differ = (a.y ^ parity) | (a.w ^ parity) | (b.y ^ parity) | (b.w ^ parity);
+            else
+                differ = (a.w ^ parity) | (b.w ^ parity);
+            if (__all_sync(0xffffffffu, !act || static_cast<int32_t>(differ) >= 0)) break;
+            if (++spins > SPIN_LIMIT) {
+                if (lane == 0) raise_status(status, ST_TIMEOUT);
+                break;
+            }
+        }
+        uint32_t pos = 0;
+        if (act && c == 0) {  // free the unit, then claim its place (units may leave in any order)
+            asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(u.fill + p))),
+                         "r"((~e & 0x8000u) << 9)
+                         : "memory");
+            pos = atomicAdd(&u.cur[p], F);
+        }
+        pos = __shfl_sync(0xffffffffu, pos, static_cast<int>(lane - c)) + c * U::CH;
+        if (act) {
+            if constexpr (TW == 2) {
+                a.y &= 0x7fffffffu;
+                a.w &= 0x7fffffffu;
+                b.y &= 0x7fffffffu;
+            } else {
+                a.w &= 0x7fffffffu;
+            }
+            b.w &= 0x7fffffffu;
+            uint32_t* g = out + static_cast<size_t>(pos) * TW;
+            if (pos + U::CH > out_cap) {
+                raise_status(status, ST_INTERNAL);
+            } else if ((static_cast<uint32_t>(reinterpret_cast<uintptr_t>(g)) & 31u) == 0) {
+                if (u.keep) st_global_v8_keep(g, a, b, ((pos + U::CH) & (4 * U::CH - 1)) != 0 ? u.keep : u.done);
+                else st_global_v8(g, a, b);
+            } else if constexpr (TW == 2) {  // half-sector groups (W = 2), or a caller's buffer on 16 bytes
+                reinterpret_cast<uint2*>(g)[0] = make_uint2(a.x, a.y);
+                reinterpret_cast<uint2*>(g)[1] = make_uint2(a.z, a.w);
+                reinterpret_cast<uint2*>(g)[2] = make_uint2(b.x, b.y);
+                reinterpret_cast<uint2*>(g)[3] = make_uint2(b.z, b.w);
+            } else {
+                reinterpret_cast<uint4*>(g)[0] = a;
+                reinterpret_cast<uint4*>(g)[1] = b;
+            }
+        }
+    }
+    // last, so that a store held up by memory holds up no slot or unit
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        bool direct = ok[v] && (old[v] & WCU_COUNT) >= F;
+        if constexpr (KEEP) {
+            const uint32_t bal = __ballot_sync(0xffffffffu, direct);
+            const uint32_t at = n_late + __popc(bal & ((1u << lane) - 1u));
+            if (direct && at < WCU_LATE) {
+                sts_tuple<TW>(u.late + at * TW, w[v], w[v][TW - 1]);
+                u.late_d[at] = static_cast<uint16_t>(dv[v]);
+                direct = false;
+            }
+            n_late = min(n_late + __popc(bal), static_cast<uint32_t>(WCU_LATE));
+        }
+        if (direct) {
+            const uint32_t pos = atomicSub(&u.back[dv[v]], 1u) - 1u;
+            if (pos < out_cap)
+                store_words<TW>(out + static_cast<size_t>(pos) * TW, w[v]);
+            else
+                raise_status(status, ST_INTERNAL);
+        }
+    }
+    __syncwarp();
+}
+
+// Places up to 32 of the warp's late tuples.
+template <typename K>
+__device__ __forceinline__ void wcu_late(const WcUnits<K>& u, uint32_t& n_late, uint32_t* __restrict__ out,
+                                         uint32_t out_cap, uint32_t* __restrict__ status)
+{
+    constexpr int TW = WcUnits<K>::TW;
+    const uint32_t first = n_late > 32u ? n_late - 32u : 0u;
+    const uint32_t at = first + (threadIdx.x & 31);
+    uint32_t w[1][TW], dv[1] = {0u};
+    const bool ok[1] = {at < n_late};
+#pragma unroll
+    for (int i = 0; i < TW; ++i) w[0][i] = ok[0] ? u.late[at * TW + i] : 0u;
+    if (ok[0]) dv[0] = u.late_d[at];
+    __syncwarp();
+    n_late = first;
+    wcu_put<K, 1, false>(u, n_late, w, dv, ok, out, out_cap, status);
+}
+
+// One round of a warp: its tuples, then late ones once 32 have gathered.
+template <typename K, int V>
+__device__ __forceinline__ void wcu_place(const WcUnits<K>& u, uint32_t& n_late,
+                                          const uint32_t (&w)[V][TupleTraits<K>::WORDS], const uint32_t (&dv)[V],
+                                          const bool (&ok)[V], uint32_t* __restrict__ out, uint32_t out_cap,
+                                          uint32_t* __restrict__ status)
+{
+    wcu_put<K, V, true>(u, n_late, w, dv, ok, out, out_cap, status);
+    if (n_late >= 32u) wcu_late<K>(u, n_late, out, out_cap, status);
+}
+
+// End of an item: every unit's remaining tuples at its front cursor, padding
+// (at most W - 1 tuples) between them and the back cursor.
+template <typename K>
+__device__ __forceinline__ void wcu_finish(const WcUnits<K>& u, uint32_t& n_late, int P, uint32_t W,
+                                           uint32_t* __restrict__ out, uint32_t out_cap,
+                                           uint32_t* __restrict__ status)
+{
+    constexpr int TW = WcUnits<K>::TW;
+    while (n_late > 0u) wcu_late<K>(u, n_late, out, out_cap, status);
+    __syncthreads();
+    const uint32_t F = 1u << u.logF, span = 2u * (F > W ? F : W);  // slots, then padding
+    const uint32_t all = static_cast<uint32_t>(P) * span;          // P * span <= 2^17
+    for (uint32_t i = threadIdx.x; i < all; i += blockDim.x) {
+        const uint32_t p = i / span, s = i & (span - 1u);
+        const uint32_t n = u.fill[p] & WCU_COUNT, at = u.cur[p], end = u.back[p];
+        if (s == 0 && (n >= F || end - at - n >= W || end > out_cap)) raise_status(status, ST_INTERNAL);
+        if (n < F && at + s < end && s < n + W && end <= out_cap) {
+            uint32_t t[TW];
+#pragma unroll
+            for (int j = 0; j < TW; ++j) t[j] = 0u;
+            if (s < n) {
+#pragma unroll
+                for (int j = 0; j < TW; ++j) t[j] = u.buf[(static_cast<size_t>(p) << u.logF) * TW + s * TW + j];
+                t[TW - 1] &= 0x7fffffffu;
+            } else {
+                t[TW - 1] = static_cast<uint32_t>(PAD_ROW);
+            }
+            store_words<TW>(out + static_cast<size_t>(at + s) * TW, t);
+        }
+    }
+    __syncthreads();
+}
+
 // Scatter of a raw key column (row = key index).  V keys per thread per
+// round (whole 16-byte vectors), the next two rounds' vectors loaded while
+// the current round is placed; the warps of the CTA run on their own.
+template <typename K, int THREADS, int V, bool HASHD, bool HEAVY>
+__global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __restrict__ keys, int64_t n,
+                                                                  int64_t chunk, int32_t n_items, DigitFn f,
+                                                                  int32_t P, int32_t logF, int32_t W, int32_t ipg,
+                                                                  const int64_t* __restrict__ offsets,
+                                                                  uint32_t* __restrict__ out, uint32_t out_cap,
+                                                                  uint32_t* __restrict__ status,
+                                                                  typename HeavyArg<HEAVY>::type hs, HeavyOut ho)
+{
+    constexpr int TW = TupleTraits<K>::WORDS;
+    constexpr int VN = Vec16<K>::N;
+    constexpr int NV = V / VN;  // vectors per thread per round
+    static_assert(V % VN == 0, "V must be whole vectors");
+    constexpr int ROUND = THREADS * V;
+    extern __shared__ __align__(128) uint8_t smem[];
+    WcUnits<K> wc;
+    wc.bind(smem, P, logF, V);
+    uint32_t n_late = 0;
+    HeavyTable heavy;
+    if constexpr (HEAVY) {
+        // after the units and the lists, on a 16-byte boundary (slots are
+        // read as 16-byte words)
+        heavy.bind(smem + ((WcUnits<K>::bytes(P, logF, THREADS, V) + 15) & ~size_t(15)));
+        heavy.build<K>(hs, ho.heavy_row);  // ends with a barrier
+    }
+    const int lane = threadIdx.x & 31;
+
+    __shared__ unsigned long long s_hbase;  // heavy pairs of the items before this one
+    __shared__ uint32_t s_hcur;             // heavy pairs of this item so far
+    for (int32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+        if constexpr (HEAVY) {
+            if (threadIdx.x < 32) {
+                unsigned long long sum = 0;
+                for (int j = threadIdx.x; j < item; j += 32) sum += ho.item_count[j];
+                for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+                if (threadIdx.x == 0) {
+                    s_hbase = sum;
+                    s_hcur = 0;
+                }
+            }
+        }
+        const int64_t* seg = offsets + seg_base(item, ipg, P);  // partition p's segment: [seg[p * ipg], seg[p * ipg + 1])
+        wcu_begin<K>(wc, P, [&](int p) { return seg[static_cast<int64_t>(p) * ipg]; },
+                     [&](int p) { return seg[static_cast<int64_t>(p) * ipg + 1]; });
+        int64_t lo = static_cast<int64_t>(item) * chunk;
+        const int64_t hi = lo + chunk < n ? lo + chunk : n;
+        if (lo > hi) lo = hi;
+        const K* kp = keys + lo;
+        const uint32_t len = static_cast<uint32_t>(hi - lo);
+        const uint32_t row0 = static_cast<uint32_t>(lo);
+
+        // element e of vector j of this thread in the round at offset b:
+        //   b + (j * THREADS + threadIdx.x) * VN + e
+        auto load_round = [&](uint32_t b, K (&dst)[NV][VN]) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                const uint32_t at = b + (static_cast<uint32_t>(j) * THREADS + threadIdx.x) * VN;
+                if (at + VN <= len) {
+                    load_vec16<K>(kp + at, dst[j]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < VN; ++e) dst[j][e] = at + e < len ? kp[at + e] : K(0);
+                }
+            }
+        };
+        K nxt[NV][VN];
+        if (len > 0) load_round(0, nxt);
+        for (uint32_t b = 0; b < len; b += ROUND) {
+            K cur[NV][VN];
+#pragma unroll
+            for (int j = 0; j < NV; ++j)
+#pragma unroll
+                for (int e = 0; e < VN; ++e) cur[j][e] = nxt[j][e];
+            if (b + ROUND < len) load_round(b + ROUND, nxt);
+            const bool full = b + ROUND <= len;
+
+            uint32_t w[V][TW];
+            uint32_t dv[V];  // the tuple's partition
+            bool ok[V];
+#pragma unroll
+            for (int j = 0; j < NV; ++j)
+#pragma unroll
+                for (int e = 0; e < VN; ++e) {
+                    const int v = j * VN + e;
+                    const uint32_t at = b + (static_cast<uint32_t>(j) * THREADS + threadIdx.x) * VN + e;
+                    ok[v] = full || at < len;
+                    const K k = cur[j][e];
+                    tuple_words<K>(w[v], k, static_cast<int32_t>(row0 + at));
+                    uint32_t d;
+                    if constexpr (HASHD) {
+                        const uint32_t h = sizeof(K) == 4 ? w[v][0] : w[v][TW - 2];
+                        d = (h >> f.shift) & f.mask;
+                    } else {
+                        d = static_cast<uint32_t>(static_cast<uint64_t>(k) >> f.shift) & f.mask;
+                    }
+                    dv[v] = d;
+                }
+            if constexpr (HEAVY) {
+                // heavy probe keys: out of the partitions, matched here
+                int32_t hb[V];
+                int c = 0;
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    hb[v] = -1;
+                    if (ok[v]) {
+                        const HeavyHit e = heavy.find(static_cast<K>(cur[v / VN][v % VN]));
+                        if (e.idx >= 0) {
+                            ok[v] = false;
+                            hb[v] = e.row;
+                            c += hb[v] >= 0 ? 1 : 0;
+                        }
+                    }
+                }
+                int incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const int tot = __shfl_sync(0xffffffffu, incl, 31);
+                if (tot > 0) {
+                    uint32_t base = 0;
+                    if (lane == 31) base = atomicAdd(&s_hcur, static_cast<uint32_t>(tot));
+                    base = __shfl_sync(0xffffffffu, base, 31);
+                    if (ho.out_build) {
+                        long long pos = static_cast<long long>(s_hbase) + base + (incl - c);
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            if (hb[v] >= 0) {
+                                if (pos < ho.capacity) {
+                                    ho.out_build[pos] = hb[v];
+                                    ho.out_probe[pos] = static_cast<int32_t>(w[v][TW - 1]);
+                                } else {
+                                    raise_status(status, ST_CAPACITY);
+                                }
+                                ++pos;
+                            }
+                        }
+                    }
+                }
+            }
+            wcu_place<K, V>(wc, n_late, w, dv, ok, out, out_cap, status);
+        }
+        wcu_finish<K>(wc, n_late, P, static_cast<uint32_t>(W), out, out_cap, status);
+    }
+}
+
+// The same scatter with wc_place, for fan-outs whose units and cursors do not
+// fit shared memory (8192 partitions of half-sector groups).  V keys per thread per
 // round (whole 16-byte vectors), the next two rounds' vectors loaded while
 // the current round is processed.  Per partition the CTA keeps a buffer of
 // cap tuples (whole groups of W), a fill count and an output cursor.
 template <typename K, int THREADS, int V, int W, bool HASHD, bool HEAVY>
-__global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __restrict__ keys, int64_t n,
+__global__ void __launch_bounds__(THREADS, 1) scatter_rounds_kernel(const K* __restrict__ keys, int64_t n,
                                                                   int64_t chunk, int32_t n_items, DigitFn f,
                                                                   int32_t P, int32_t cap,
                                                                   const int64_t* __restrict__ offsets,
@@ -750,24 +1215,26 @@ __global__ void __launch_bounds__(HIST_THREADS) hist_tuples_kernel(const uint32_
 }
 
 // Pass-two scatter: the pass-one tuples of each item, placed by the next
-// hash bits through the same write-combining buffers as the first pass.
+// hash bits through the same write-combining units as the first pass.
 // VT tuples per thread per round, the next round's loaded ahead.
-template <typename K, int THREADS, int VT, int W>
+template <typename K, int THREADS, int VT>
 __global__ void __launch_bounds__(THREADS, 1) scatter_tuples_kernel(const uint32_t* __restrict__ in, Pass2Items it,
                                                                     int32_t n_items, DigitFn f, int32_t P,
-                                                                    int32_t cap, const int64_t* __restrict__ offsets,
+                                                                    int32_t logF, int32_t W,
+                                                                    const int64_t* __restrict__ offsets,
                                                                     uint32_t* __restrict__ out, uint32_t out_cap,
                                                                     uint32_t* __restrict__ status)
 {
-    constexpr int TW = WcTraits<K, W>::TW;
+    constexpr int TW = TupleTraits<K>::WORDS;
     constexpr int ROUND = THREADS * VT;
     extern __shared__ __align__(128) uint8_t smem[];
-    uint32_t* buf = reinterpret_cast<uint32_t*>(smem);
-    const WcState fc = WcState::at(buf + static_cast<size_t>(P) * cap * TW, P);
+    WcUnits<K> wc;
+    wc.bind(smem, P, logF, VT);
+    uint32_t n_late = 0;
     for (int32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
-        for (int p = threadIdx.x; p < P; p += THREADS)
-            fc.init(p, static_cast<int>(offsets[static_cast<int64_t>(p) * n_items + item]));
-        __syncthreads();
+        const int64_t* seg = offsets + item;
+        wcu_begin<K>(wc, P, [&](int p) { return seg[static_cast<int64_t>(p) * n_items]; },
+                     [&](int p) { return seg[static_cast<int64_t>(p) * n_items + 1]; });
         int64_t lo, hi;
         pass2_range(it, item, lo, hi);
         uint32_t nw[VT][TW];
@@ -792,10 +1259,9 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_tuples_kernel(const uint32
                 dv[v] = (tuple_hash<K>(w[v]) >> f.shift) & f.mask;
             }
             if (b + ROUND < hi) load_round(b + ROUND);
-            wc_place<K, W, VT>(w, dv, ok, buf, cap, fc, out, out_cap, status);
+            wcu_place<K, VT>(wc, n_late, w, dv, ok, out, out_cap, status);
         }
-        wc_finish<K, W>(P, buf, cap, fc, out, out_cap, offsets, n_items, item, status);
-        __syncthreads();
+        wcu_finish<K>(wc, n_late, P, static_cast<uint32_t>(W), out, out_cap, status);
     }
 }
 
@@ -842,24 +1308,24 @@ __global__ void __launch_bounds__(HIST_THREADS) hist_seg_kernel(const SegItem* _
 
 // Write-combining scatter of the items (persistent grid; buffers sized for
 // the largest partition count of the batch, Pmax).
-template <typename K, int THREADS, int VT, int W>
+template <typename K, int THREADS, int VT>
 __global__ void __launch_bounds__(THREADS, 1) scatter_seg_kernel(const SegItem* __restrict__ items, int32_t n_items,
-                                                                 int32_t Pmax, int32_t cap,
+                                                                 int32_t Pmax, int32_t logF, int32_t W,
                                                                  const int64_t* __restrict__ offsets,
                                                                  uint32_t* __restrict__ out, uint32_t out_cap,
                                                                  uint32_t* __restrict__ status)
 {
-    constexpr int TW = WcTraits<K, W>::TW;
+    constexpr int TW = TupleTraits<K>::WORDS;
     constexpr int ROUND = THREADS * VT;
     extern __shared__ __align__(128) uint8_t smem[];
-    uint32_t* buf = reinterpret_cast<uint32_t*>(smem);
-    const WcState fc = WcState::at(buf + static_cast<size_t>(Pmax) * cap * TW, Pmax);
+    WcUnits<K> wc;
+    wc.bind(smem, Pmax, logF, VT);
+    uint32_t n_late = 0;
     for (int32_t i = blockIdx.x; i < n_items; i += gridDim.x) {
         const SegItem it = items[i];
         const int64_t* off = offsets + it.cnt_base;
-        for (int p = threadIdx.x; p < it.P; p += THREADS)
-            fc.init(p, static_cast<int>(off[static_cast<int64_t>(p) * it.seg_items + it.item]));
-        __syncthreads();
+        wcu_begin<K>(wc, it.P, [&](int p) { return off[static_cast<int64_t>(p) * it.seg_items + it.item]; },
+                     [&](int p) { return off[static_cast<int64_t>(p) * it.seg_items + it.item + 1]; });
         const K* keys = static_cast<const K*>(it.keys);
         K nk[VT];
         auto load_round = [&](int64_t b) {
@@ -882,10 +1348,9 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_seg_kernel(const SegItem* 
                 dv[v] = (tuple_hash<K>(w[v]) >> it.f.shift) & it.f.mask;
             }
             if (b + ROUND < it.hi) load_round(b + ROUND);
-            wc_place<K, W, VT>(w, dv, ok, buf, cap, fc, out, out_cap, status);
+            wcu_place<K, VT>(wc, n_late, w, dv, ok, out, out_cap, status);
         }
-        wc_finish<K, W>(it.P, buf, cap, fc, out, out_cap, off, it.seg_items, it.item, status);
-        __syncthreads();
+        wcu_finish<K>(wc, n_late, it.P, static_cast<uint32_t>(W), out, out_cap, status);
     }
 }
 
