@@ -311,8 +311,11 @@ pj_status pj_partition(const void* keys, int64_t n, int32_t key_bytes, const pj_
 
 /* ---- batches of joins (no reference counterpart: the reference runs one
  * join per process) --------------------------------------------------------
- * Joins whose build side fits one shared-memory table skip partitioning: one
- * persistent kernel drains a (join, probe chunk) work queue over all of
+ * Joins with unique build keys of up to 2^22 rows are joined through hash
+ * tables in L2, a group of joins at a time: one launch builds the group's
+ * tables, one probes them, every match written at an exact position of its
+ * join's output (large_batched = 1).  Of the others, joins whose build side
+ * fits one shared-memory table skip partitioning: one persistent kernel drains a (join, probe chunk) work queue over all of
  * them, writing each join's pairs densely to its own output.  Larger joins
  * (up to 2^10 partitions each) are partitioned together -- one histogram,
  * one scan and one scatter launch over both key columns of all of them --
@@ -325,7 +328,8 @@ typedef struct pj_batch_config {
     int32_t direct_chunk;      /* probe rows per direct work item (>= 1024) */
     int32_t direct_max_build;  /* joins with at most this many build rows go direct (<= 40960) */
     int32_t large_bits_delta;  /* added to the default radix bits of the partitioned joins */
-    int32_t large_batched;     /* 1: partitioned joins run together (above); 0: one after another */
+    int32_t large_batched;     /* 1: joins through tables in L2, partitioned joins together (above);
+                                  0: direct joins, the others one after another */
 } pj_batch_config;
 
 /* Defaults for a key width. */

@@ -42,7 +42,7 @@ constexpr int HEAVY_SAMPLES = 1 << 16;     // probe keys the planner samples
 constexpr int HEAVY_MIN_SAMPLES = 32;      // a heavy key holds >= 1/2048 of the sample
 constexpr int64_t HEAVY_MIN_PROBE = 1 << 20;  // smaller probe sides: no heavy-key path
 constexpr double HEAVY_MIN_SHARE = 0.5;       // share of the probe rows the heavy keys must hold
-constexpr int64_t GLOBAL_MAX_BUILD = 1 << 22;     // build rows of a join by one table in L2
+constexpr int64_t GLOBAL_MAX_BUILD = GT_MAX_BUILD;  // build rows of a join by one table in L2
 constexpr int64_t GLOBAL_SPARSE_BUILD = 1 << 20;  // up to here its table has four slots a row
 constexpr int64_t GROUP_BYTES = int64_t(256) << 20;  // tuples of one item group (pj_partition.cuh)
 constexpr size_t LEARN_BYTES = 4096;          // features, activations and scores of the learned planner

@@ -40,6 +40,7 @@ constexpr int GT_STEPS = 4;                 // steps of a CTA (one where the pro
 constexpr uint32_t GT_MAX_BUCKETS = 1u << 13;  // buckets an insert or a lookup tries
 constexpr uint32_t GT_LONG = 32;            // repeated keys: ranges beyond this are walked by the warp
 constexpr int GT_ROW_BITS = 22;             // 8-byte keys: row bits of a slot
+constexpr int64_t GT_MAX_BUILD = int64_t(1) << GT_ROW_BITS;  // build rows of a table
 constexpr int GT_STAGE = 2048;              // repeated keys: pairs a CTA stages for whole-run stores
 
 struct GlobalOut {
@@ -153,12 +154,14 @@ __global__ void __launch_bounds__(GT_THREADS) gt_build_kernel(const K* __restric
 
 // This thread's two probe keys: rows 2t, 2t + 1 of the tile, one load
 // streamed past L1 and marked evict-first in L2 (the table should stay).
+// vec: the column starts on a 16-byte boundary (batches take any).
 template <typename K>
-__device__ __forceinline__ void gt_load_pair(const K* __restrict__ keys, uint32_t n, uint32_t row0, K (&k)[GT_U])
+__device__ __forceinline__ void gt_load_pair(const K* __restrict__ keys, bool vec, uint32_t n, uint32_t row0,
+                                             K (&k)[GT_U])
 {
     uint64_t pol;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    if (row0 + 1 < n) {
+    if (vec && row0 + 1 < n) {
         if constexpr (sizeof(K) == 4) {
             uint32_t x, y;
             asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;"
@@ -176,7 +179,7 @@ __device__ __forceinline__ void gt_load_pair(const K* __restrict__ keys, uint32_
         }
     } else {
         k[0] = row0 < n ? keys[row0] : K(0);
-        k[1] = K(0);
+        k[1] = row0 + 1 < n ? keys[row0 + 1] : K(0);
     }
 }
 
@@ -259,17 +262,17 @@ __device__ __forceinline__ void gt_store_pair(const GlobalOut& o, unsigned long 
 // low, and all steps share one reservation -- with one per 512 rows every
 // third stall was its barrier (3 M x 10 M 8-byte keys: 112 us).
 template <typename K, int STEPS>
-__global__ void __launch_bounds__(GT_THREADS, STEPS == 1 ? 2048 / GT_THREADS : 1536 / GT_THREADS)
-    gt_probe_kernel(const K* __restrict__ pkeys, uint32_t n, const K* __restrict__ bkeys,
-                    const uint32_t* __restrict__ table, uint32_t nb, GlobalOut o)
+__device__ __forceinline__ void gt_probe_block(const K* __restrict__ pkeys, bool vec, uint32_t n,
+                                               const K* __restrict__ bkeys, const uint32_t* __restrict__ table,
+                                               uint32_t nb, const GlobalOut& o, uint32_t block_row)
 {
     using S = GtSlots<K>;
     __shared__ unsigned long long s_warp[GT_THREADS / 32 + 2];
-    const uint32_t row0 = blockIdx.x * (STEPS * GT_TILE) + threadIdx.x * GT_U;
+    const uint32_t row0 = block_row + threadIdx.x * GT_U;
     int32_t m[STEPS][GT_U];
     uint32_t again = 0;  // bit j * GT_U + u: that row needs the whole search
     K k[GT_U], nk[GT_U];
-    gt_load_pair<K>(pkeys, n, row0, nk);
+    gt_load_pair<K>(pkeys, vec, n, row0, nk);
 #pragma unroll
     for (int j = 0; j < STEPS; ++j) {
         const uint32_t r0 = row0 + j * GT_TILE;
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(GT_THREADS, STEPS == 1 ? 2048 / GT_THREADS : 1
             h[u] = hash_key(k[u]);
             gt_load_bucket(table, gt_bucket(h[u], nb), w[u]);
         }
-        if (j + 1 < STEPS) gt_load_pair<K>(pkeys, n, r0 + GT_TILE, nk);
+        if (j + 1 < STEPS) gt_load_pair<K>(pkeys, vec, n, r0 + GT_TILE, nk);
 #pragma unroll
         for (int u = 0; u < GT_U; ++u) {
             bool full;
@@ -335,6 +338,69 @@ __global__ void __launch_bounds__(GT_THREADS, STEPS == 1 ? 2048 / GT_THREADS : 1
             if (m[j][u] >= 0) gt_store_pair(o, base + off[j][u], m[j][u], row0 + j * GT_TILE + u);
 }
 
+template <typename K, int STEPS>
+__global__ void __launch_bounds__(GT_THREADS, STEPS == 1 ? 2048 / GT_THREADS : 1536 / GT_THREADS)
+    gt_probe_kernel(const K* __restrict__ pkeys, uint32_t n, const K* __restrict__ bkeys,
+                    const uint32_t* __restrict__ table, uint32_t nb, GlobalOut o)
+{
+    gt_probe_block<K, STEPS>(pkeys, true, n, bkeys, table, nb, o, blockIdx.x * (STEPS * GT_TILE));
+}
+
+// ---- batches -----------------------------------------------------------------
+// Many joins, a group at a time: the tables of a group lie side by side in one
+// region that stays in L2, one launch builds them and one probes them.  Every
+// CTA takes one item {join, first row} of a table made when the batch was
+// prepared.
+struct GtJob {
+    const void* build;
+    const void* probe;
+    int32_t* out_build;  // nullptr: count only
+    int32_t* out_probe;
+    int64_t capacity;
+    unsigned long long* count;
+    uint32_t n_build, n_probe;
+    uint32_t nb;            // buckets
+    uint32_t first_bucket;  // in the group's region
+    uint32_t vec;           // the probe column starts on 16 bytes
+    uint32_t pad;
+};
+struct GtItem {
+    uint32_t job;
+    uint32_t row0;
+};
+constexpr uint32_t GT_BUILD_ITEM = 4 * GT_THREADS;      // build rows of an item (GT_THREADS in a small batch)
+constexpr uint32_t GT_PROBE_ITEM = GT_STEPS * GT_TILE;  // probe rows of an item (GT_TILE in a small batch)
+
+template <typename K>
+__global__ void __launch_bounds__(GT_THREADS) gt_batch_build_kernel(const GtJob* __restrict__ jobs,
+                                                                    const GtItem* __restrict__ items,
+                                                                    uint32_t item_rows, uint32_t* region,
+                                                                    uint32_t* status)
+{
+    const GtItem it = items[blockIdx.x];
+    const GtJob* __restrict__ J = jobs + it.job;
+    const K* keys = static_cast<const K*>(J->build);
+    uint32_t* table = region + static_cast<size_t>(J->first_bucket) * 8;
+    const uint32_t n = J->n_build, nb = J->nb;
+    if (it.row0 == 0 && threadIdx.x == 0) *J->count = 0;
+#pragma unroll 1
+    for (uint32_t i = it.row0 + threadIdx.x; i < n && i < it.row0 + item_rows; i += GT_THREADS)
+        gt_insert<K>(keys, table, nb, keys[i], i, status);
+}
+
+template <typename K, int STEPS>
+__global__ void __launch_bounds__(GT_THREADS, STEPS == 1 ? 2048 / GT_THREADS : 1536 / GT_THREADS)
+    gt_batch_probe_kernel(const GtJob* __restrict__ jobs, const GtItem* __restrict__ items,
+                          const uint32_t* __restrict__ region, uint32_t* status)
+{
+    const GtItem it = items[blockIdx.x];
+    const GtJob* __restrict__ J = jobs + it.job;
+    const GlobalOut o{J->out_build, J->out_probe, J->capacity, J->count, status};
+    gt_probe_block<K, STEPS>(static_cast<const K*>(J->probe), J->vec != 0, J->n_probe,
+                                static_cast<const K*>(J->build), region + static_cast<size_t>(J->first_bucket) * 8,
+                                J->nb, o, it.row0);
+}
+
 // ---- repeated build keys ---------------------------------------------------
 
 template <typename K>
@@ -351,7 +417,7 @@ __global__ void __launch_bounds__(GT_THREADS) gt_count_kernel(const K* __restric
 // CTA lie one after another, the CTAs in whatever order they come (one
 // atomic each instead of a scan over all of them).
 constexpr int GT_ALLOC = 8;  // buckets per thread
-__global__ void __launch_bounds__(GT_THREADS) gt_alloc_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
+static __global__ void __launch_bounds__(GT_THREADS) gt_alloc_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
                                                               uint2* __restrict__ range, unsigned long long* cursor)
 {
     __shared__ unsigned long long s_warp[GT_THREADS / 32 + 2];
@@ -399,7 +465,7 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
     const uint32_t row0 = blockIdx.x * GT_TILE + threadIdx.x * GT_U;
     K k[GT_U];
     uint32_t h[GT_U], lo[GT_U], hi[GT_U], c[GT_U];
-    gt_load_pair<K>(pkeys, n, row0, k);
+    gt_load_pair<K>(pkeys, true, n, row0, k);
 #pragma unroll
     for (int u = 0; u < GT_U; ++u) {
         h[u] = hash_key(k[u]);
