@@ -238,6 +238,12 @@ pj_status pj_inner_join_events(const pj_join_desc* desc, const pj_plan* plan, pj
  * PJ_ERR_TIMEOUT or PJ_ERR_INTERNAL), then clears it. */
 pj_status pj_check(void* workspace, pj_stream stream);
 
+/* pj_check, and in *count (host) the int64 at byte PJ_WORKSPACE_COUNT of the
+ * workspace, both by one copy.  The library only clears that word; a join
+ * whose pj_output.count points to it leaves its match count there. */
+#define PJ_WORKSPACE_COUNT 8
+pj_status pj_check_count(void* workspace, int64_t* count, pj_stream stream);
+
 /* Diagnostics of the bounded device waits (no reference counterpart: the
  * reference's only bounded loop is the build insert's attempt counter,
  * hash_join_kernels.cuh:104-127).  Runs the build side's decoupled

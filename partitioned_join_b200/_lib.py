@@ -14,6 +14,7 @@ DIGIT_RAW, DIGIT_HASH = 0, 1
 SLOT_FAST, SLOT_REF = 0, 1
 SPLIT_HASH, SPLIT_POSITION = 0, 1
 TABLE_BUCKET, TABLE_OPEN, TABLE_COMPACT, TABLE_EXACT = 0, 1, 2, 3
+WORKSPACE_COUNT = 8               # PJ_WORKSPACE_COUNT
 NOALLOC_SCRATCH_BYTES = 64 << 20  # PJ_NOALLOC_SCRATCH_BYTES
 MAX_HEAVY = 256                   # PJ_MAX_HEAVY
 STAGES = ["build_hist", "build_scan", "build_scatter", "build_pass2", "probe_hist", "probe_scan", "probe_scatter",
@@ -90,6 +91,7 @@ SIGNATURES = {
                                             _SZ, _P, ctypes.POINTER(ctypes.c_void_p)]),
     "pj_join_count": (ctypes.c_int, [ctypes.POINTER(JoinDesc), ctypes.POINTER(Plan), _P, _P, _SZ, _P]),
     "pj_check": (ctypes.c_int, [_P, _P]),
+    "pj_check_count": (ctypes.c_int, [_P, ctypes.POINTER(_I64), _P]),
     "pj_diag_scan_timeout": (ctypes.c_int, [ctypes.POINTER(JoinDesc), ctypes.POINTER(Plan), _P, _SZ, _I64,
                                             ctypes.c_uint32, _P]),
     "pj_inner_join_noalloc": (ctypes.c_int, [ctypes.POINTER(JoinDesc), ctypes.POINTER(Plan), ctypes.POINTER(Output), _P]),

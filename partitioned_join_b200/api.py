@@ -110,6 +110,17 @@ def alloc_workspace(nbytes: int, device) -> torch.Tensor:
     return ws
 
 
+def _count(desc: JoinDesc, plan: Plan, ws: torch.Tensor, ws_bytes: int) -> int:
+    """pj_join_count with the count in the workspace's head."""
+    st = _stream_ptr(None)
+    p = ctypes.c_void_p(ws.data_ptr())
+    n = ctypes.c_int64(0)
+    check(lib().pj_join_count(ctypes.byref(desc), ctypes.byref(plan),
+                              ctypes.c_void_p(ws.data_ptr() + _lib.WORKSPACE_COUNT), p, ws_bytes, st), "pj_join_count")
+    check(lib().pj_check_count(p, ctypes.byref(n), st), "pj_join_count")
+    return n.value
+
+
 class Joiner:
     """Reusable join context: workspace and output buffers sized once for a
     (sizes, plan), so repeated joins allocate nothing (bench and batch use)."""
@@ -133,20 +144,17 @@ class Joiner:
         dev = self.build_keys.device
         self.ws_bytes = workspace_size(self.desc, self.plan)
         self.ws = alloc_workspace(self.ws_bytes, dev)
+        # the match count lies in the workspace's head: one copy reads it with the status
+        self.count = self.ws[_lib.WORKSPACE_COUNT:_lib.WORKSPACE_COUNT + 8].view(torch.int64)
         if capacity is None:
             capacity = self.desc.n_probe if unique_build_keys else self._count()
         self.capacity = int(capacity)
         self.build_row = torch.empty(max(self.capacity, 1), dtype=torch.int32, device=dev)
         self.probe_row = torch.empty(max(self.capacity, 1), dtype=torch.int32, device=dev)
-        self.count = torch.zeros(1, dtype=torch.int64, device=dev)
+        self.count.zero_()
 
     def _count(self) -> int:
-        cnt = torch.zeros(1, dtype=torch.int64, device=self.build_keys.device)
-        st = _stream_ptr(None)
-        check(lib().pj_join_count(ctypes.byref(self.desc), ctypes.byref(self.plan), ctypes.c_void_p(cnt.data_ptr()),
-                                  ctypes.c_void_p(self.ws.data_ptr()), self.ws_bytes, st), "pj_join_count")
-        check(lib().pj_check(ctypes.c_void_p(self.ws.data_ptr()), st), "pj_join_count")
-        return int(cnt.item())
+        return _count(self.desc, self.plan, self.ws, self.ws_bytes)
 
     def launch(self, stream=None) -> None:
         """Enqueue the join on the stream (asynchronous)."""
@@ -186,9 +194,16 @@ class Joiner:
         """Synchronise and return the device-side status (pj_check)."""
         return lib().pj_check(ctypes.c_void_p(self.ws.data_ptr()), _stream_ptr(stream))
 
+    def status_count(self, stream=None) -> Tuple[int, int]:
+        """Synchronise; the device-side status and the match count."""
+        n = ctypes.c_int64(0)
+        st = lib().pj_check_count(ctypes.c_void_p(self.ws.data_ptr()), ctypes.byref(n), _stream_ptr(stream))
+        return st, n.value
+
     def result(self, stream=None) -> Tuple[torch.Tensor, torch.Tensor]:
-        st = self.status(stream)
-        n = int(self.count.item())
+        return self._pairs(*self.status_count(stream))
+
+    def _pairs(self, st: int, n: int) -> Tuple[torch.Tensor, torch.Tensor]:
         if st == _lib.ERR_CAPACITY:
             raise PJError(st, f"need capacity {n}, have {self.capacity}")
         check(st, "pj_inner_join")
@@ -204,12 +219,12 @@ def partitioned_join(build_keys: torch.Tensor, probe_keys: torch.Tensor, unique_
     (inner_join_cpu.hpp:24-107) carried as row indices."""
     j = Joiner(build_keys, probe_keys, unique_build_keys, plan, capacity)
     j.launch(stream)
-    st = j.status(stream)
+    st, n = j.status_count(stream)
     if st == _lib.ERR_CAPACITY and capacity is None:
-        n = int(j.count.item())
         j = Joiner(build_keys, probe_keys, unique_build_keys, j.plan, n)
         j.launch(stream)
-    return j.result(stream)
+        st, n = j.status_count(stream)
+    return j._pairs(st, n)
 
 
 def partitioned_join_payload(build_keys: torch.Tensor, probe_keys: torch.Tensor,
@@ -231,8 +246,8 @@ def partitioned_join_payload(build_keys: torch.Tensor, probe_keys: torch.Tensor,
     out.probe_payload_out = pp.data_ptr() if pp is not None else None
     check(lib().pj_inner_join(ctypes.byref(desc), ctypes.byref(j.plan), ctypes.byref(out),
                               ctypes.c_void_p(j.ws.data_ptr()), j.ws_bytes, _stream_ptr(stream)), "pj_inner_join")
-    check(j.status(stream), "pj_inner_join")
-    n = int(j.count.item())
+    st, n = j.status_count(stream)
+    check(st, "pj_inner_join")
     return (j.build_row[:n], j.probe_row[:n], pb[:n] if pb is not None else None,
             pp[:n] if pp is not None else None)
 
@@ -384,13 +399,7 @@ def join_count(build_keys: torch.Tensor, probe_keys: torch.Tensor, unique_build_
     if plan is None:
         plan = plan_default(d.n_build, d.n_probe, d.key_bytes, unique_build_keys)
     nb = workspace_size(d, plan)
-    ws = alloc_workspace(nb, build_keys.device)
-    cnt = torch.zeros(1, dtype=torch.int64, device=build_keys.device)
-    st = _stream_ptr(None)
-    check(lib().pj_join_count(ctypes.byref(d), ctypes.byref(plan), ctypes.c_void_p(cnt.data_ptr()),
-                              ctypes.c_void_p(ws.data_ptr()), nb, st), "pj_join_count")
-    check(lib().pj_check(ctypes.c_void_p(ws.data_ptr()), st), "pj_join_count")
-    return int(cnt.item())
+    return _count(d, plan, alloc_workspace(nb, build_keys.device), nb)
 
 
 def plan_exact(build_keys: torch.Tensor, probe_keys: torch.Tensor, unique_build_keys: bool = True,

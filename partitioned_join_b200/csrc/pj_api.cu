@@ -1386,19 +1386,36 @@ pj_status pj_join_count(const pj_join_desc* d, const pj_plan* plan, int64_t* cou
                          StageEvents());
 }
 
-pj_status pj_check(void* ws, pj_stream stream)
+pj_status pj_check_count(void* ws, int64_t* count, pj_stream stream)
 {
     if (!ws) return PJ_ERR_WORKSPACE;
-    PJ_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
-    uint32_t st = 0;
-    PJ_CUDA(cudaMemcpy(&st, ws, sizeof(st), cudaMemcpyDeviceToHost));
-    const uint32_t zero = 0;
-    PJ_CUDA(cudaMemcpy(ws, &zero, sizeof(zero), cudaMemcpyHostToDevice));
-    if (st & ST_INTERNAL) return PJ_ERR_INTERNAL;
-    if (st & ST_TIMEOUT) return PJ_ERR_TIMEOUT;
-    if (st & ST_OVERFLOW) return PJ_ERR_OVERFLOW;
-    if (st & ST_CAPACITY) return PJ_ERR_CAPACITY;
+    if (!count) return PJ_ERR_INVALID;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    struct {
+        uint32_t status, unused;
+        int64_t count;
+    } head{};
+    static_assert(sizeof(head) == 16 && PJ_WORKSPACE_COUNT == 8, "the workspace's first 16 bytes");
+    PJ_CUDA(cudaMemcpyAsync(&head, ws, sizeof(head), cudaMemcpyDeviceToHost, st));
+    PJ_CUDA(cudaStreamSynchronize(st));
+    *count = head.count;
+    const uint32_t v = head.status;
+    if (v) {  // (a clean status needs no clearing copy)
+        const uint32_t zero = 0;
+        PJ_CUDA(cudaMemcpyAsync(ws, &zero, sizeof(zero), cudaMemcpyHostToDevice, st));
+        PJ_CUDA(cudaStreamSynchronize(st));
+    }
+    if (v & ST_INTERNAL) return PJ_ERR_INTERNAL;
+    if (v & ST_TIMEOUT) return PJ_ERR_TIMEOUT;
+    if (v & ST_OVERFLOW) return PJ_ERR_OVERFLOW;
+    if (v & ST_CAPACITY) return PJ_ERR_CAPACITY;
     return PJ_OK;
+}
+
+pj_status pj_check(void* ws, pj_stream stream)
+{
+    int64_t count = 0;
+    return pj_check_count(ws, &count, stream);
 }
 
 pj_status pj_diag_scan_timeout(const pj_join_desc* d, const pj_plan* plan, void* ws, size_t ws_bytes,

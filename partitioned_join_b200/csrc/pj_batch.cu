@@ -614,7 +614,7 @@ pj_status pj_batch_check(void* ws, pj_stream stream)
     uint32_t v = 0;
     if (cudaMemcpy(&v, ws, sizeof(v), cudaMemcpyDeviceToHost) != cudaSuccess) return PJ_ERR_CUDA;
     const uint32_t zero = 0;
-    if (cudaMemcpy(ws, &zero, sizeof(zero), cudaMemcpyHostToDevice) != cudaSuccess) return PJ_ERR_CUDA;
+    if (v && cudaMemcpy(ws, &zero, sizeof(zero), cudaMemcpyHostToDevice) != cudaSuccess) return PJ_ERR_CUDA;
     if (v & ST_INTERNAL) return PJ_ERR_INTERNAL;
     if (v & ST_TIMEOUT) return PJ_ERR_TIMEOUT;
     if (v & ST_OVERFLOW) return PJ_ERR_OVERFLOW;
