@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(512) global_hist_kernel(const K* __restrict__ 
 // Single-pass exclusive scan with decoupled look-back (Merrill & Garland,
 // "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016).
 // out[i] = sum_{j<i} r(in[j]), out[m] = total, with r(x) = x rounded up to a
-// multiple of round_to.  Tiles are claimed through an atomic counter, so a
+// multiple of round_to (a power of two).  Tiles are claimed through an atomic counter, so a
 // tile's predecessors are always already running; the look-back spin is
 // bounded all the same.  tile_state and tile_counter must be zero.
 constexpr int SCAN_THREADS = 512;
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) lookback_scan_kernel(const TIn* 
     for (int j = 0; j < SCAN_ITEMS; ++j) {
         const int64_t idx = base + j;
         int64_t x = idx < m ? static_cast<int64_t>(in[idx]) : 0;
-        if (round_to > 1) x = (x + round_to - 1) / round_to * round_to;
+        x = (x + round_to - 1) & ~static_cast<int64_t>(round_to - 1);
         v[j] = x;
         sum += x;
     }
@@ -278,34 +278,42 @@ __global__ void __launch_bounds__(SCAN_THREADS) lookback_scan_kernel(const TIn* 
     const int64_t block_total = s_warp[SCAN_THREADS / 32 - 1];
     const int64_t thread_excl = incl - sum + (warp > 0 ? s_warp[warp - 1] : 0);
 
-    if (threadIdx.x == 0) {
+    // Warp 0 looks back 32 tiles at a time: lane l at tile `at - l`.  The
+    // aggregates up to the nearest published prefix are this tile's offset.
+    // (One thread stepping back tile by tile took most of the kernel: 2^18
+    // counters 12 us, 606 K counters 20 us.)
+    if (warp == 0) {
         int64_t excl = 0;
         if (tile == wait.withhold_tile) {
             // publishes nothing: its successors' waits run out
         } else if (tile == 0) {
-            st_release_u64(&tile_state[0], TS_PREFIX | static_cast<uint64_t>(block_total));
+            if (lane == 0) st_release_u64(&tile_state[0], TS_PREFIX | static_cast<uint64_t>(block_total));
         } else {
-            st_release_u64(&tile_state[tile], TS_AGG | static_cast<uint64_t>(block_total));
-            int64_t i = tile - 1;
+            if (lane == 0) st_release_u64(&tile_state[tile], TS_AGG | static_cast<uint64_t>(block_total));
             uint32_t spins = 0;
-            while (i >= 0) {
-                const uint64_t s = ld_acquire_u64(&tile_state[i]);
-                const uint64_t flag = s & ~TS_VALUE;
-                if (flag == 0) {
+            for (int64_t at = tile - 1;;) {
+                const uint64_t s = at >= lane ? ld_acquire_u64(&tile_state[at - lane]) : TS_PREFIX;
+                const uint32_t published = __ballot_sync(0xffffffffu, (s & ~TS_VALUE) != 0);
+                const uint32_t prefixes = __ballot_sync(0xffffffffu, (s & ~TS_VALUE) == TS_PREFIX);
+                const uint32_t upto = prefixes ? (prefixes & -prefixes) * 2u - 1u : 0xffffffffu;  // lanes that count
+                if ((published & upto) != upto) {
                     if (++spins > wait.spin_limit) {
-                        raise_status(status, ST_TIMEOUT);
+                        if (lane == 0) raise_status(status, ST_TIMEOUT);
                         break;
                     }
                     __nanosleep(32);
                     continue;
                 }
-                excl += static_cast<int64_t>(s & TS_VALUE);
-                if (flag == TS_PREFIX) break;
-                --i;
+                int64_t v32 = (upto >> lane) & 1u ? static_cast<int64_t>(s & TS_VALUE) : 0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v32 += __shfl_xor_sync(0xffffffffu, v32, o);
+                excl += v32;
+                if (prefixes) break;
+                at -= 32;
             }
-            st_release_u64(&tile_state[tile], TS_PREFIX | static_cast<uint64_t>(excl + block_total));
+            if (lane == 0) st_release_u64(&tile_state[tile], TS_PREFIX | static_cast<uint64_t>(excl + block_total));
         }
-        s_excl = excl;
+        if (lane == 0) s_excl = excl;
     }
     __syncthreads();
     int64_t run = s_excl + thread_excl;
