@@ -417,12 +417,11 @@ Layout make_layout(const pj_join_desc* d, const pj_plan* p, bool grouped = true)
     L.b_tiles2_n = L.p_tiles2_n = two ? (m2 + SCAN_TILE - 1) / SCAN_TILE + 1 : 0;
     L.b_ipg = L.b_items;
     L.p_ipg = L.p_items;
-    // Groups where the join walks ranges by position in the partition: not for
-    // a second pass, COMPACT entries (which index the build range) or OPEN tables,
-    // nor for half-sector groups' own scatter.
-    if (grouped && !two && (p->table_mode == PJ_TABLE_BUCKET || p->table_mode == PJ_TABLE_EXACT) &&
-        sector_wc(d->key_bytes, p->wc_tuples)) {
-        L.b_ipg = items_per_group(L.b_items, L.b_chunk, d->key_bytes);
+    // Groups where the join walks a partition range by range: not for a second
+    // pass, OPEN tables or half-sector groups (their own scatter), nor the
+    // build side of COMPACT tables, whose entries index one range.
+    if (grouped && !two && p->table_mode != PJ_TABLE_OPEN && sector_wc(d->key_bytes, p->wc_tuples)) {
+        if (p->table_mode != PJ_TABLE_COMPACT) L.b_ipg = items_per_group(L.b_items, L.b_chunk, d->key_bytes);
         L.p_ipg = items_per_group(L.p_items, L.p_chunk, d->key_bytes);
     }
     L.b_groups = (L.b_items + L.b_ipg - 1) / L.b_ipg;
@@ -769,7 +768,7 @@ pj_status launch_join_g(const JoinArgs& a, cudaStream_t st)
 template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF>
 pj_status launch_join_t(const JoinArgs& a, cudaStream_t st)
 {
-    if constexpr (TABLE == TABLE_BUCKET || TABLE == TABLE_EXACT)
+    if constexpr (TABLE != TABLE_OPEN)
         if (a.b_groups > 1 || a.p_groups > 1) return launch_join_g<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, MAX_GROUPS>(a, st);
     if (a.b_groups != 1 || a.p_groups != 1) return PJ_ERR_INVALID;
     return launch_join_g<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, 1>(a, st);

@@ -118,8 +118,20 @@ __global__ void __launch_bounds__(512) heavy_rows_kernel(const K* __restrict__ k
     HeavyTable t;
     t.bind(smem);
     t.build<K>(hs, nullptr);
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    // four keys in flight a thread
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    for (; i + 3 * stride < n; i += 4 * stride) {
+        K k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) k[u] = __ldg(keys + i + u * stride);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const HeavyHit e = t.find(k[u]);
+            if (e.idx >= 0) heavy_row[e.idx] = static_cast<int32_t>(i + u * stride);
+        }
+    }
+    for (; i < n; i += stride) {
         const HeavyHit e = t.find(keys[i]);
         if (e.idx >= 0) heavy_row[e.idx] = static_cast<int32_t>(i);
     }

@@ -795,6 +795,41 @@ __device__ __forceinline__ void wcu_place(const WcUnits<K>& u, uint32_t& n_late,
     if (n_late >= 32u) wcu_late<K>(u, n_late, out, out_cap, status);
 }
 
+// A round of which few tuples are to be placed (most are heavy keys): they
+// join the late list, and 32 at a time are placed together.  Placing them
+// where they are costs a whole round's instructions for, at Zipf 1.5, every
+// seventh lane (2^26 int64 probe rows, 105 heavy keys: 551 -> 453 us).
+template <typename K, int V>
+__device__ __forceinline__ void wcu_place_few(const WcUnits<K>& u, uint32_t& n_late,
+                                              const uint32_t (&w)[V][TupleTraits<K>::WORDS], const uint32_t (&dv)[V],
+                                              const bool (&ok)[V], uint32_t* __restrict__ out, uint32_t out_cap,
+                                              uint32_t* __restrict__ status)
+{
+    constexpr int TW = WcUnits<K>::TW;
+    uint32_t bal[V], total = 0;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        bal[v] = __ballot_sync(0xffffffffu, ok[v]);
+        total += __popc(bal[v]);
+    }
+    if (total > 20u * V) {
+        wcu_place<K, V>(u, n_late, w, dv, ok, out, out_cap, status);
+        return;
+    }
+    const uint32_t lt = (1u << (threadIdx.x & 31)) - 1u;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        if (n_late + __popc(bal[v]) > WCU_LATE) wcu_late<K>(u, n_late, out, out_cap, status);
+        const uint32_t at = n_late + __popc(bal[v] & lt);
+        if (ok[v]) {
+            sts_tuple<TW>(u.late + at * TW, w[v], w[v][TW - 1]);
+            u.late_d[at] = static_cast<uint16_t>(dv[v]);
+        }
+        n_late += __popc(bal[v]);
+        __syncwarp();
+    }
+}
+
 // End of an item: every unit's remaining tuples at its front cursor, padding
 // (at most W - 1 tuples) between them and the back cursor.
 template <typename K>
@@ -828,6 +863,63 @@ __device__ __forceinline__ void wcu_finish(const WcUnits<K>& u, uint32_t& n_late
     __syncthreads();
 }
 
+// The heavy ones among a thread's V probe keys leave the partitions (ok =
+// false), and their pairs go to the output: after the pairs of earlier items
+// (first) and of this item so far (*done, in shared memory).  Positions go by
+// key index, then lane, so every store instruction writes one run (lane by
+// lane, each lane's pairs together, the same scatter took 453 us, not 414).
+// Whole warp.
+template <typename K, int V>
+__device__ __forceinline__ void heavy_take(const HeavyTable& heavy, const K (&key)[V], const uint32_t (&row)[V],
+                                           bool (&ok)[V], unsigned long long first, uint32_t* done, const HeavyOut& ho,
+                                           uint32_t* __restrict__ status)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    int32_t hb[V];
+    uint32_t off[V], total = 0;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        hb[v] = -1;
+        if (ok[v]) {
+            const HeavyHit e = heavy.find(key[v]);
+            if (e.idx >= 0) {
+                ok[v] = false;
+                hb[v] = e.row;
+            }
+        }
+        __syncwarp();
+        const uint32_t bal = __ballot_sync(0xffffffffu, hb[v] >= 0);
+        off[v] = total + __popc(bal & lt);
+        total += __popc(bal);
+    }
+    if (total == 0) return;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(done, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (!ho.out_build) return;
+    const long long pos = static_cast<long long>(first) + base;
+    if (pos + total <= ho.capacity) {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (hb[v] >= 0) {
+                __stcs(ho.out_build + pos + off[v], hb[v]);
+                __stcs(ho.out_probe + pos + off[v], static_cast<int32_t>(row[v]));
+            }
+    } else {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (hb[v] >= 0) {
+                if (pos + off[v] < ho.capacity) {
+                    ho.out_build[pos + off[v]] = hb[v];
+                    ho.out_probe[pos + off[v]] = static_cast<int32_t>(row[v]);
+                } else {
+                    raise_status(status, ST_CAPACITY);
+                }
+            }
+    }
+}
+
 // Scatter of a raw key column (row = key index).  V keys per thread per
 // round (whole 16-byte vectors), the next two rounds' vectors loaded while
 // the current round is placed; the warps of the CTA run on their own.
@@ -856,7 +948,6 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __res
         heavy.bind(smem + ((WcUnits<K>::bytes(P, logF, THREADS, V) + 15) & ~size_t(15)));
         heavy.build<K>(hs, ho.heavy_row);  // ends with a barrier
     }
-    const int lane = threadIdx.x & 31;
 
     __shared__ unsigned long long s_hbase;  // heavy pairs of the items before this one
     __shared__ uint32_t s_hcur;             // heavy pairs of this item so far
@@ -929,50 +1020,17 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __res
                     dv[v] = d;
                 }
             if constexpr (HEAVY) {
-                // heavy probe keys: out of the partitions, matched here
-                int32_t hb[V];
-                int c = 0;
+                K key[V];
+                uint32_t row[V];
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
-                    hb[v] = -1;
-                    if (ok[v]) {
-                        const HeavyHit e = heavy.find(static_cast<K>(cur[v / VN][v % VN]));
-                        if (e.idx >= 0) {
-                            ok[v] = false;
-                            hb[v] = e.row;
-                            c += hb[v] >= 0 ? 1 : 0;
-                        }
-                    }
+                    key[v] = static_cast<K>(cur[v / VN][v % VN]);
+                    row[v] = w[v][TW - 1];
                 }
-                int incl = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += y;
-                }
-                const int tot = __shfl_sync(0xffffffffu, incl, 31);
-                if (tot > 0) {
-                    uint32_t base = 0;
-                    if (lane == 31) base = atomicAdd(&s_hcur, static_cast<uint32_t>(tot));
-                    base = __shfl_sync(0xffffffffu, base, 31);
-                    if (ho.out_build) {
-                        long long pos = static_cast<long long>(s_hbase) + base + (incl - c);
-#pragma unroll
-                        for (int v = 0; v < V; ++v) {
-                            if (hb[v] >= 0) {
-                                if (pos < ho.capacity) {
-                                    ho.out_build[pos] = hb[v];
-                                    ho.out_probe[pos] = static_cast<int32_t>(w[v][TW - 1]);
-                                } else {
-                                    raise_status(status, ST_CAPACITY);
-                                }
-                                ++pos;
-                            }
-                        }
-                    }
-                }
+                heavy_take<K, V>(heavy, key, row, ok, s_hbase, &s_hcur, ho, status);
             }
-            wcu_place<K, V>(wc, n_late, w, dv, ok, out, out_cap, status);
+            if constexpr (HEAVY) wcu_place_few<K, V>(wc, n_late, w, dv, ok, out, out_cap, status);
+            else wcu_place<K, V>(wc, n_late, w, dv, ok, out, out_cap, status);
         }
         wcu_finish<K>(wc, n_late, P, static_cast<uint32_t>(W), out, out_cap, status);
     }
@@ -1007,7 +1065,6 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_rounds_kernel(const K* __r
         heavy.bind(smem + heavy_table_offset(P, cap * TW));
         heavy.build<K>(hs, ho.heavy_row);  // ends with a barrier
     }
-    const int lane = threadIdx.x & 31;
 
     __shared__ unsigned long long s_hbase;  // heavy pairs of the items before this one
     __shared__ uint32_t s_hcur;             // heavy pairs of this item so far
@@ -1084,48 +1141,14 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_rounds_kernel(const K* __r
                     dv[v] = d;
                 }
             if constexpr (HEAVY) {
-                // heavy probe keys: out of the partitions, matched here
-                int32_t hb[V];
-                int c = 0;
+                K key[V];
+                uint32_t row[V];
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
-                    hb[v] = -1;
-                    if (ok[v]) {
-                        const HeavyHit e = heavy.find(static_cast<K>(cur[v / VN][v % VN]));
-                        if (e.idx >= 0) {
-                            ok[v] = false;
-                            hb[v] = e.row;
-                            c += hb[v] >= 0 ? 1 : 0;
-                        }
-                    }
+                    key[v] = static_cast<K>(cur[v / VN][v % VN]);
+                    row[v] = w[v][TW - 1];
                 }
-                int incl = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += y;
-                }
-                const int tot = __shfl_sync(0xffffffffu, incl, 31);
-                if (tot > 0) {
-                    uint32_t base = 0;
-                    if (lane == 31) base = atomicAdd(&s_hcur, static_cast<uint32_t>(tot));
-                    base = __shfl_sync(0xffffffffu, base, 31);
-                    if (ho.out_build) {
-                        long long pos = static_cast<long long>(s_hbase) + base + (incl - c);
-#pragma unroll
-                        for (int v = 0; v < V; ++v) {
-                            if (hb[v] >= 0) {
-                                if (pos < ho.capacity) {
-                                    ho.out_build[pos] = hb[v];
-                                    ho.out_probe[pos] = static_cast<int32_t>(w[v][TW - 1]);
-                                } else {
-                                    raise_status(status, ST_CAPACITY);
-                                }
-                                ++pos;
-                            }
-                        }
-                    }
-                }
+                heavy_take<K, V>(heavy, key, row, ok, s_hbase, &s_hcur, ho, status);
             }
             wc_place<K, W, V>(w, dv, ok, buf, cap, fc, out, out_cap, status);
         }
