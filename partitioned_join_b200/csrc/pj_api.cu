@@ -26,15 +26,13 @@ namespace {
 // Fixed kernel configurations.
 constexpr int SC_THREADS = 1024;
 constexpr int SC_V32 = 4, SC_V64 = 2;  // keys per thread per round (one 16-byte vector)
-#ifndef PJ_JOIN_THREADS
-// 24 warps of up to 85 registers: the 1024-thread form (64 registers) spilled
-// in the probe loop; 2^27 x 2^27 int32 join 2.43 -> 2.37 ms, 2^26 x 2^28
-// int64 4.37 -> 3.73 ms (512, 640, 896 threads all measured slower; 832
-// threads: int32 0.997 -> 1.007 ms, int64 1.95 -> 1.93 ms)
-constexpr int JN_THREADS = 768;
-#else
-constexpr int JN_THREADS = PJ_JOIN_THREADS;
-#endif
+// Working threads of a join CTA (and one planner warp beside them).  24 warps
+// of 72 registers for 4-byte keys, 23 of 80 for 8-byte keys, whose probe spills
+// at 72 (25 warps leave one quarter of the SM seven): 2^24 x 2^26 int64 628 ->
+// 597 us, 2^27 x 2^27 int32 with 23 warps 1.09 -> 1.13 ms.
+template <typename K>
+constexpr int jn_threads() { return sizeof(K) == 4 ? 768 : 736; }
+constexpr int JN_BLOCK_MAX = 768 + 32;
 constexpr int MAX_SPLIT_LOG2 = 6;
 constexpr int MAX_BUCKET_CAP = 65535;  // 16-bit bucket ends
 constexpr int MAX_JOIN_CTAS_PER_SM = 4;
@@ -333,7 +331,7 @@ int join_ctas_per_sm(int key_bytes, const pj_plan* p)
 {
     const size_t smem = join_smem(key_bytes, p->table_mode, p->table_capacity);
     const int by_smem = static_cast<int>((smem_limit() + 1024) / std::max<size_t>(smem + 1024, 1));
-    const int by_threads = 2048 / JN_THREADS;
+    const int by_threads = 2048 / JN_BLOCK_MAX;
     return std::max(1, std::min({MAX_JOIN_CTAS_PER_SM, by_smem, by_threads}));
 }
 
@@ -384,12 +382,14 @@ int scatter_items(const pj_plan* p) { return sm_count() * std::max(1, p->scatter
 int64_t part_capacity(int64_t n, int P, int items, int W) { return n + static_cast<int64_t>(items) * P * (W - 1) + W; }
 
 // Items per group (pj_partition.cuh) of a column of n_items chunks: groups of
-// at most GROUP_BYTES of tuples, at most MAX_GROUPS of them; one group while
-// the column is not much larger.
-int items_per_group(int n_items, int64_t chunk, int key_bytes)
+// at most GROUP_BYTES of tuples, at most MAX_GROUPS of them.  One group where
+// groups gain the scatter less than ranges cost the join: 4096 partitions gain
+// from 512 MB on (2^27 int32 keys: 0.84 -> 0.61 ms for 0.04 ms), fewer ones only
+// past 1 GB (2048 partitions of 2^28 int64 keys 2.27 -> 2.01 ms, of 2^26 none).
+int items_per_group(int n_items, int64_t chunk, int key_bytes, int P)
 {
     const int64_t bytes = chunk * tuple_words(key_bytes) * 4;
-    if (bytes * n_items <= 2 * GROUP_BYTES) return n_items;
+    if (bytes * n_items <= (P >= 4096 ? 2 : 5) * GROUP_BYTES) return n_items;
     const int64_t fit = std::max<int64_t>(1, GROUP_BYTES / bytes);
     return static_cast<int>(std::max<int64_t>(fit, (n_items + MAX_GROUPS - 1) / MAX_GROUPS));
 }
@@ -421,8 +421,8 @@ Layout make_layout(const pj_join_desc* d, const pj_plan* p, bool grouped = true)
     // pass, OPEN tables or half-sector groups (their own scatter), nor the
     // build side of COMPACT tables, whose entries index one range.
     if (grouped && !two && p->table_mode != PJ_TABLE_OPEN && sector_wc(d->key_bytes, p->wc_tuples)) {
-        if (p->table_mode != PJ_TABLE_COMPACT) L.b_ipg = items_per_group(L.b_items, L.b_chunk, d->key_bytes);
-        L.p_ipg = items_per_group(L.p_items, L.p_chunk, d->key_bytes);
+        if (p->table_mode != PJ_TABLE_COMPACT) L.b_ipg = items_per_group(L.b_items, L.b_chunk, d->key_bytes, L.P1);
+        L.p_ipg = items_per_group(L.p_items, L.p_chunk, d->key_bytes, L.P1);
     }
     L.b_groups = (L.b_items + L.b_ipg - 1) / L.b_ipg;
     L.p_groups = (L.p_items + L.p_ipg - 1) / L.p_ipg;
@@ -743,14 +743,14 @@ pj_status launch_scatter(const K* keys, int64_t n, int64_t chunk, int items, Dig
 template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF, int NG>
 pj_status launch_join_g(const JoinArgs& a, cudaStream_t st)
 {
-    auto* kern = join_kernel<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, JN_THREADS, NG>;
+    auto* kern = join_kernel<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, jn_threads<K>(), NG>;
     const size_t smem = JoinSmem<K, TABLE>::bytes(a.cap, a.nb_log2);
     PJ_CUDA(set_smem(kern, smem));
     int per_sm = 0;
-    PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, JN_THREADS, smem));
+    PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, jn_threads<K>() + 32, smem));
     per_sm = std::min(std::max(per_sm, 1), MAX_JOIN_CTAS_PER_SM);
     const int grid = std::min(sm_count() * per_sm, a.max_ctas);
-    kern<<<grid, JN_THREADS, smem, st>>>(a);
+    kern<<<grid, jn_threads<K>() + 32, smem, st>>>(a);
     PJ_CUDA(cudaGetLastError());
     // fix-up: dense output and the true count
     const int fix_threads = std::min(MAX_FIXUP_CTAS, (grid + 31) / 32 * 32);
@@ -1890,14 +1890,14 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
         const size_t smem = JoinSmem<K, TABLE_BUCKET>::bytes(a.cap, a.nb_log2);
         PJ_CUDA(set_smem(kern, smem));
         int per_sm = 0;
-        PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, JN_THREADS, smem));
+        PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, jn_threads<K>() + 32, smem));
         per_sm = std::min(std::max(per_sm, 1), MAX_JOIN_CTAS_PER_SM);
-        kern<<<sm_count() * per_sm, JN_THREADS, smem, st>>>(a);
+        kern<<<sm_count() * per_sm, jn_threads<K>() + 32, smem, st>>>(a);
         PJ_CUDA(cudaGetLastError());
         return PJ_OK;
     };
-    if (lb.unique) return launch(join_kernel<K, TABLE_BUCKET, true, true, false, JN_THREADS, 1, true>);
-    return launch(join_kernel<K, TABLE_BUCKET, false, false, false, JN_THREADS, 1, true>);
+    if (lb.unique) return launch(join_kernel<K, TABLE_BUCKET, true, true, false, jn_threads<K>(), 1, true>);
+    return launch(join_kernel<K, TABLE_BUCKET, false, false, false, jn_threads<K>(), 1, true>);
 }
 
 }  // namespace

@@ -112,7 +112,15 @@ constexpr int32_t PAD_ROW = -1;
 // ---------------------------------------------------------------------------
 // Exclusive scan, in place, of the 16-bit counts packed two per word in
 // w[0 .. nwords).  Totals stay below 65536.  Ends with __syncthreads().
-template <int THREADS>
+// BAR > 0: the threads [0, THREADS) of a larger block, by that named barrier.
+template <int THREADS, int BAR>
+__device__ __forceinline__ void part_sync()
+{
+    if constexpr (BAR == 0) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(THREADS) : "memory");
+}
+
+template <int THREADS, int BAR = 0>
 __device__ __forceinline__ void scan_u16_pairs(uint32_t* w, int nwords, uint32_t* s_warp)
 {
     // an odd run length: the lanes of a warp then walk 32 different banks
@@ -132,7 +140,7 @@ __device__ __forceinline__ void scan_u16_pairs(uint32_t* w, int nwords, uint32_t
         if (lane >= o) incl += y;
     }
     if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
+    part_sync<THREADS, BAR>();
     if (warp == 0) {
         uint32_t x = lane < THREADS / 32 ? s_warp[lane] : 0u;
 #pragma unroll
@@ -142,7 +150,7 @@ __device__ __forceinline__ void scan_u16_pairs(uint32_t* w, int nwords, uint32_t
         }
         if (lane < THREADS / 32) s_warp[lane] = x;
     }
-    __syncthreads();
+    part_sync<THREADS, BAR>();
     uint32_t run = incl - sum + (warp > 0 ? s_warp[warp - 1] : 0u);
     for (int i = a; i < b; ++i) {
         const uint32_t x = w[i];
@@ -150,7 +158,7 @@ __device__ __forceinline__ void scan_u16_pairs(uint32_t* w, int nwords, uint32_t
         w[i] = (run & 0xffffu) | ((run + c0) << 16);
         run += c0 + c1;
     }
-    __syncthreads();
+    part_sync<THREADS, BAR>();
 }
 
 // Bounded spin: iterations before a wait gives up and raises ST_TIMEOUT.

@@ -437,7 +437,7 @@ constexpr int JOIN_BU = 4;       // build tuples in flight per thread
 constexpr uint32_t JOIN_STEP = 128;  // tuples a warp takes at a time (32 lanes x JOIN_U = JOIN_BU)
 static_assert(JOIN_U * 32 == JOIN_STEP && JOIN_BU * 32 == JOIN_STEP, "a step is U tuples a lane");
 
-// One work item.  Warp 0 works out the next one while the current one probes,
+// One work item.  A warp of its own works out the next one while the current one probes,
 // so an item starts without a chain of dependent global loads (item ->
 // partition -> offsets).
 struct ItemMeta {
@@ -508,7 +508,7 @@ struct JoinSmem {
 };
 
 template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF, int THREADS, int NG, bool BATCH = false>
-__global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
+__global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
 {
     using TV = TupleView<K>;
     using Cmp = typename TV::Cmp;
@@ -517,6 +517,10 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
     constexpr int NWARPS = THREADS / 32;
     const int lane = threadIdx.x & 31;
     constexpr int U = JOIN_U;
+    // The block's last warp works out the next item while the others build and
+    // probe: inside their loop its code cost them the registers they spilled.
+    const bool planner = threadIdx.x >= THREADS;
+    constexpr int BAR_WORK = 1, BAR_BUILT = 2;  // named barriers: the working warps; they and the planner
 
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* table = smem;
@@ -544,7 +548,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
     const int64_t total_items = a.item_off[a.P];
     const bool write_out = a.out_build != nullptr;
 
-    // Warp 0: item `it` as the next item.  prev_p: the build tuples are fetched
+    // The planner warp: item `it` as the next item.  prev_p: the build tuples are fetched
     // into L2 unless that partition's are there already (COMPACT tables: see
     // the call).
     auto load_meta = [&](int64_t it, int prev_p) {
@@ -616,7 +620,7 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
             s_nmeta = m;
         }
     };
-    if (threadIdx.x < 32) {
+    if (planner) {
         int64_t it = 0;
         if (lane == 0) {
             s_q = 0;
@@ -753,12 +757,11 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
     };
     for (;;) {
         __syncthreads();
-        if (threadIdx.x < 32) {
+        if (planner) {
             if (lane == 0) {
                 s_item = s_next;
                 s_meta = s_nmeta;
                 if constexpr (BATCH) s_jout = s_njout;
-                s_next = static_cast<int64_t>(atomicAdd(a.queue, 1u));  // claim the next item early
             }
             if (lane < NG) {
                 s_bst.last[lane] = s_nbst.last[lane];
@@ -772,23 +775,35 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
         __syncthreads();
         const int64_t item = s_item;
         if (item >= total_items || item >= a.max_items) break;
-        const int p = s_meta.p;
+        if (planner) {
+            // the head of the probe chunk streams into L2 while the table is built
+            if (lane < NG) {
+                const int64_t head = PROBE_PREFETCH_BYTES / (TV::WORDS * 4);
+                const int64_t left = head - (lane > 0 ? static_cast<int64_t>(s_qst.last[lane - 1]) * JOIN_STEP : 0);
+                const int64_t n = s_qst.n[lane] < left ? s_qst.n[lane] : left;
+                if (n > 0)
+                    prefetch_l2_stream(a.probe_tuples + static_cast<int64_t>(s_qst.start[lane]) * TV::WORDS,
+                                       n * TV::WORDS * 4, stream_pol);
+            }
+            int64_t next = 0;
+            if (lane == 0) s_next = next = static_cast<int64_t>(atomicAdd(a.queue, 1u));  // claim the next item early
+            next = __shfl_sync(0xffffffffu, next, 0);
+            // The next item's build side streams into L2 while this item probes,
+            // so the next build's count pass reads L2 (BUCKET tables: 8% at
+            // 2^25; EXACT tables: 2^27 x 2^27 int32 join 1.72 -> 1.59 ms).  Not
+            // for COMPACT tables: their fingerprint checks re-read build tuples
+            // and the prefetched ranges were evicted before use (0.83 GB more
+            // DRAM reads at 2^27 x 2^27, no time gained).
+            asm volatile("bar.sync %0, %1;" ::"n"(BAR_BUILT), "n"(THREADS + 32) : "memory");
+            if (next < total_items && next < a.max_items) load_meta(next, s_meta.p);
+            continue;
+        }
         const uint32_t piece = static_cast<uint32_t>(s_meta.piece);
         const int sbits = s_meta.sbits;
         const int dbits = s_meta.dbits;
         if constexpr (BATCH) jout = s_jout;
         const int skip = dbits + sbits;
         const int piece_shift = 32 - (sbits > 0 ? sbits : 1);
-
-        // the head of the probe chunk streams into L2 while the table is built
-        if (threadIdx.x < NG) {
-            const int64_t head = PROBE_PREFETCH_BYTES / (TV::WORDS * 4);
-            const int64_t left = head - (lane > 0 ? static_cast<int64_t>(s_qst.last[lane - 1]) * JOIN_STEP : 0);
-            const int64_t n = s_qst.n[lane] < left ? s_qst.n[lane] : left;
-            if (n > 0)
-                prefetch_l2_stream(a.probe_tuples + static_cast<int64_t>(s_qst.start[lane]) * TV::WORDS,
-                                   n * TV::WORDS * 4, stream_pol);
-        }
 
         auto in_piece = [&](uint32_t h) -> bool {
             if (!HASH_SPLIT || sbits == 0) return true;
@@ -815,14 +830,14 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
             // an entry's 16-bit index cannot address this range: the planner avoids it
             if (threadIdx.x == 0) raise_status(a.status, ST_OVERFLOW);
             skip_item = true;
-            __syncthreads();
+            part_sync<THREADS, BAR_WORK>();
         } else if constexpr (TABLE != TABLE_OPEN) {
             // bucket directory: 16-bit counts of bucket b at index b + 1; after
             // the scan and the place pass index b holds the start of bucket b
             // and index b + 1 its end
             for (int i = threadIdx.x; i <= NB / 2; i += THREADS) ends[i] = 0u;
             if (threadIdx.x == 0) s_nbuild = 0;
-            __syncthreads();
+            part_sync<THREADS, BAR_WORK>();
             // pass 1: count per bucket; the next batch of loads is issued
             // before the current one is counted
             int mine = 0;
@@ -862,12 +877,12 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
             }
             mine = __reduce_add_sync(0xffffffffu, mine);
             if (lane == 0 && mine) atomicAdd(&s_nbuild, mine);
-            __syncthreads();
+            part_sync<THREADS, BAR_WORK>();
             if (s_nbuild > a.cap) {  // the planner sizes pieces to fit; flag and skip
                 if (threadIdx.x == 0) raise_status(a.status, ST_OVERFLOW);
                 skip_item = true;
             } else {
-                scan_u16_pairs<THREADS>(ends, NB / 2 + 1, s_warp);
+                scan_u16_pairs<THREADS, BAR_WORK>(ends, NB / 2 + 1, s_warp);
                 // pass 2: place
                 StepCursor<NG, TV::WORDS> cur;
                 for (uint32_t st = warp; st < b_total; st += NWARPS) {
@@ -898,13 +913,13 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                     }
                 }
             }
-            __syncthreads();
+            part_sync<THREADS, BAR_WORK>();
         } else {
             for (int i = threadIdx.x; i < a.cap; i += THREADS) {
                 if constexpr (sizeof(K) == 4) reinterpret_cast<uint2*>(table)[i] = make_uint2(0u, EMPTY_ROW);
                 else orows[i] = EMPTY_ROW;
             }
-            __syncthreads();
+            part_sync<THREADS, BAR_WORK>();
             StepCursor<NG, TV::WORDS> cur;
             for (uint32_t s4 = warp; s4 < b_total * JOIN_BU; s4 += NWARPS) {
                 uint32_t h = 0;
@@ -932,20 +947,11 @@ __global__ void __launch_bounds__(THREADS, 1) join_kernel(JoinArgs a)
                     }
                 }
             }
-            __syncthreads();
+            part_sync<THREADS, BAR_WORK>();
         }
 
-        // the next item's build side streams into L2 while this item probes,
-        // so the next build's count pass reads L2 (BUCKET tables: 8% at
-        // 2^25; EXACT tables: 2^27 x 2^27 int32 join 1.72 -> 1.59 ms).  Not
-        // for COMPACT tables: their fingerprint checks re-read build tuples
-        // and the prefetched ranges were evicted before use (0.83 GB more
-        // DRAM reads at 2^27 x 2^27, no time gained).
-        if (threadIdx.x < 32) {
-            const int64_t next = s_next;
-            if (next < total_items && next < a.max_items) load_meta(next, p);
-            __syncwarp();
-        }
+        // (the planner may fetch the next item's build side now)
+        asm volatile("bar.arrive %0, %1;" ::"n"(BAR_BUILT), "n"(THREADS + 32) : "memory");
 
         // ---- probe: warps run independently; loads run one step ahead ----
         if (!skip_item) {
