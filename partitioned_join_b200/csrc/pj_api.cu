@@ -683,16 +683,32 @@ pj_status launch_scan(const TIn* in, int64_t m, uint32_t round_to, int64_t* out,
 // (the fewer partitions, the more tuples of a round meet in one unit); -1
 // where units and cursors do not fit beside `extra` bytes.
 template <typename K>
-int unit_logf(int P, int W, int v, size_t extra)
+int unit_logf(int P, int W, int threads, int v, size_t extra)
 {
     using U = WcUnits<K>;
     int lf = U::LOG_CH;
     while ((1 << lf) < W) ++lf;
-    if (lf > U::MAX_LOGF || U::bytes(P, lf, SC_THREADS, v) + extra > smem_limit()) return -1;
+    if (lf > U::MAX_LOGF || U::bytes(P, lf, threads, v) + extra > smem_limit()) return -1;
     while (lf < U::MAX_LOGF && (static_cast<size_t>(P) << (lf + 1)) * U::TW * 4 <= (size_t(128) << 10) &&
-           U::bytes(P, lf + 1, SC_THREADS, v) + extra <= smem_limit())
+           U::bytes(P, lf + 1, threads, v) + extra <= smem_limit())
         ++lf;
     return lf;
+}
+
+template <typename K, int THREADS, bool HASHD, bool HEAVY>
+pj_status launch_scatter_units(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P, int lf, int W,
+                               int ipg, const int64_t* offsets, uint32_t* out, uint32_t cap32, uint32_t* status,
+                               const HeavyCtx& hc, cudaStream_t st)
+{
+    constexpr int V = sc_v<K>();
+    auto* kern = scatter_keys_kernel<K, THREADS, V, HASHD, HEAVY>;
+    const size_t smem = WcUnits<K>::bytes(P, lf, THREADS, V) + (HEAVY ? HeavyTable::BYTES + 16 : 0);
+    PJ_CUDA(set_smem(kern, smem));
+    typename HeavyArg<HEAVY>::type h{};
+    if constexpr (HEAVY) h = *hc.hs;
+    kern<<<items, THREADS, smem, st>>>(keys, n, chunk, items, f, P, lf, W, ipg, offsets, out, cap32, status, h, hc.out);
+    PJ_CUDA(cudaGetLastError());
+    return PJ_OK;
 }
 
 template <typename K, bool HASHD, bool HEAVY>
@@ -704,14 +720,18 @@ pj_status launch_scatter_t(const K* keys, int64_t n, int64_t chunk, int items, D
     if constexpr (HEAVY) h = *hc.hs;
     const uint32_t cap32 = static_cast<uint32_t>(std::min<int64_t>(out_cap, UINT32_MAX));
     constexpr int V = sc_v<K>();
-    const int lf = unit_logf<K>(P, W, V, HEAVY ? HeavyTable::BYTES + 16 : 0);
+    const int lf = unit_logf<K>(P, W, SC_THREADS, V, HEAVY ? HeavyTable::BYTES + 16 : 0);
     if (lf >= 0 && chunk <= static_cast<int64_t>(WCU_COUNT)) {
-        auto* kern = scatter_keys_kernel<K, SC_THREADS, V, HASHD, HEAVY>;
-        const size_t smem = WcUnits<K>::bytes(P, lf, SC_THREADS, V) + (HEAVY ? HeavyTable::BYTES + 16 : 0);
-        PJ_CUDA(set_smem(kern, smem));
-        kern<<<items, SC_THREADS, smem, st>>>(keys, n, chunk, items, f, P, lf, W, ipg, offsets, out, cap32, status, h, hc.out);
-        PJ_CUDA(cudaGetLastError());
-        return PJ_OK;
+        // 8-byte keys over 4096 partitions: two tuples a unit, and HBM takes the
+        // sectors no faster than half the warps bring them (2^28 keys 2.40 ->
+        // 2.16 ms); fewer partitions wait on the warps (2048: 434 -> 473 us), as
+        // do heavy keys (2^28 keys, 4096 partitions, Zipf 1.5: 1.56 -> 1.88 ms)
+        if constexpr (sizeof(K) == 8 && !HEAVY)
+            if (P >= 4096)
+                return launch_scatter_units<K, SC_THREADS / 2, HASHD, HEAVY>(keys, n, chunk, items, f, P, lf, W, ipg,
+                                                                             offsets, out, cap32, status, hc, st);
+        return launch_scatter_units<K, SC_THREADS, HASHD, HEAVY>(keys, n, chunk, items, f, P, lf, W, ipg, offsets, out,
+                                                                 cap32, status, hc, st);
     }
     if constexpr (sizeof(K) == 4) {  // 8192 partitions of half-sector groups
         if (W != 2 || ipg != items) return PJ_ERR_INVALID;
@@ -848,7 +868,7 @@ pj_status launch_scatter_tuples(const uint32_t* in, const Pass2Items& it, int n_
 {
     constexpr int VT = sizeof(K) == 4 ? 4 : 2;
     auto* kern = scatter_tuples_kernel<K, SC_THREADS, VT>;
-    const int lf = unit_logf<K>(P2, W, VT, 0);
+    const int lf = unit_logf<K>(P2, W, SC_THREADS, VT, 0);
     if (lf < 0) return PJ_ERR_INVALID;
     const size_t smem = WcUnits<K>::bytes(P2, lf, SC_THREADS, VT);
     PJ_CUDA(set_smem(kern, smem));
@@ -1842,7 +1862,7 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
                                    reinterpret_cast<uint64_t*>(w + lb.o_tiles), ctr + CTR_BTILE, status, st)) != PJ_OK)
         return s;
     constexpr int VT = sizeof(K) == 4 ? 4 : 2;
-    const int lf = unit_logf<K>(lb.Pmax, lb.W, VT, 0);
+    const int lf = unit_logf<K>(lb.Pmax, lb.W, SC_THREADS, VT, 0);
     if (lf < 0) return PJ_ERR_INVALID;
     const size_t ssmem = WcUnits<K>::bytes(lb.Pmax, lf, SC_THREADS, VT);
     const uint32_t out_cap = static_cast<uint32_t>(std::min<int64_t>(lb.tuples, UINT32_MAX));
