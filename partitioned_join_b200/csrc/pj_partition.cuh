@@ -555,6 +555,18 @@ __device__ __forceinline__ void wc_finish(int P, uint32_t* buf, int cap, WcState
 // registers frees the unit: the fill word moves to the other parity and
 // count 0 before the sector leaves.
 //
+// What makes this race-free: a tuple is stored and read by one scalar memory
+// operation of its size (64 or 128 bits; a vector access would be several in
+// no stated order), so parity and words are seen together; the fill word is
+// only ever touched by atomics (a plain store beside atomicAdd could be lost);
+// and the unit changes hands by them -- the release exchange that frees it,
+// after a __syncwarp behind the last lane's read, and the acquire add that
+// takes a slot -- so no read meets the next unit's tuple and no later read
+// an older one's of the same parity.  The release waits for the warp's earlier
+// sectors: 2^27 int32 keys over 4096 partitions 0.63 ms, 0.61 without it (a
+// fence a round in its place 0.65; 2^28 int64 keys 2.17, 2.15 and 2.46 ms).
+// The acquire and the scalar accesses cost nothing measurable.
+//
 // The block-wide form (three barriers per round of one vector a thread)
 // waited on shared-memory latency and barriers with half the issue slots
 // idle.  A count needs no reset bound: it grows by one per tuple of the
@@ -596,7 +608,7 @@ struct WcUnits {
         // 0.60 ms, of 2^28 int64 keys 2.94 -> 2.39 ms, 2048 of 2^26 int64 keys
         // 0.49 -> 0.43 ms (without the demotion 0.605, 2.45, 0.43).  At 2048
         // partitions of int32 keys, whose scatter waits on the SMs, the
-        // policy operands cost 4 %.
+        // policy operands cost 4 %.  (Before units were freed by a release exchange.)
         keep = done = 0;
         if (P >= (CH == 4 ? 4096 : 2048)) {
             asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
@@ -613,25 +625,62 @@ struct WcUnits {
     }
 };
 
-__device__ __forceinline__ uint4 lds_v4(const uint32_t* p)
-{
-    uint4 v;
-    asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p)))
-                 : "memory");
-    return v;
-}
-
+// A tuple in shared memory, by one scalar store and one scalar load.
 template <int TW>
 __device__ __forceinline__ void sts_tuple(uint32_t* p, const uint32_t (&w)[TW], uint32_t row)
 {
     const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
     if constexpr (TW == 2)
-        asm volatile("st.volatile.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(w[0]), "r"(row) : "memory");
-    else
-        asm volatile("st.volatile.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(row)
+        asm volatile("{ .reg .b64 t; mov.b64 t, {%1, %2}; st.relaxed.cta.shared.b64 [%0], t; }" ::"r"(a), "r"(w[0]),
+                     "r"(row)
                      : "memory");
+    else
+        asm volatile("{ .reg .b64 l, h; .reg .b128 t; mov.b64 l, {%1, %2}; mov.b64 h, {%3, %4}; mov.b128 t, {l, h}; "
+                     "st.relaxed.cta.shared.b128 [%0], t; }" ::"r"(a),
+                     "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(row)
+                     : "memory");
+}
+
+// The 16 bytes at p: two 8-byte tuples, or one of 16 bytes.
+template <int TW>
+__device__ __forceinline__ uint4 lds_tuples(const uint32_t* p)
+{
+    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+    uint4 v;
+    if constexpr (TW == 2)
+        asm volatile("{ .reg .b64 l, h; ld.relaxed.cta.shared.v2.b64 {l, h}, [%4]; mov.b64 {%0, %1}, l; "
+                     "mov.b64 {%2, %3}, h; }"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "r"(a)
+                     : "memory");
+    else
+        asm volatile("{ .reg .b64 l, h; .reg .b128 t; ld.relaxed.cta.shared.b128 t, [%4]; mov.b128 {l, h}, t; "
+                     "mov.b64 {%0, %1}, l; mov.b64 {%2, %3}, h; }"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "r"(a)
+                     : "memory");
+    return v;
+}
+
+// A slot of a unit: the fill word before this tuple.
+__device__ __forceinline__ uint32_t unit_take(uint32_t* fill)
+{
+    uint32_t old;
+    asm volatile("atom.acquire.cta.shared.add.u32 %0, [%1], 1;"
+                 : "=r"(old)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(fill)))
+                 : "memory");
+    return old;
+}
+
+// The unit is free again, with this fill word.
+__device__ __forceinline__ void unit_free(uint32_t* fill, uint32_t word)
+{
+    uint32_t old;
+    asm volatile("atom.release.cta.shared.exch.b32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(fill))), "r"(word)
+                 : "memory");
 }
 
 // Start of an item: empty units of parity 1 over slots of parity 0, cursors
@@ -664,7 +713,7 @@ __device__ __forceinline__ void wcu_put(const WcUnits<K>& u, uint32_t& n_late,
     const int lane = threadIdx.x & 31;
     uint32_t old[V];
 #pragma unroll
-    for (int v = 0; v < V; ++v) old[v] = ok[v] ? atomicAdd(&u.fill[dv[v]], 1u) : WCU_COUNT;
+    for (int v = 0; v < V; ++v) old[v] = ok[v] ? unit_take(&u.fill[dv[v]]) : WCU_COUNT;
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         const uint32_t c = old[v] & WCU_COUNT;
@@ -694,8 +743,8 @@ __device__ __forceinline__ void wcu_put(const WcUnits<K>& u, uint32_t& n_late,
         uint4 a, b;
         uint32_t spins = 0;
         for (;;) {
-            a = lds_v4(src);
-            b = lds_v4(src + 4);
+            a = lds_tuples<TW>(src);
+            b = lds_tuples<TW>(src + 4);
             uint32_t differ;
             if constexpr (TW == 2)
                 differ = (a.y ^ parity) | (a.w ^ parity) | (b.y ^ parity) | (b.w ^ parity);
@@ -707,11 +756,10 @@ __device__ __forceinline__ void wcu_put(const WcUnits<K>& u, uint32_t& n_late,
                 break;
             }
         }
+        __syncwarp();  // every lane has its sector
         uint32_t pos = 0;
         if (act && c == 0) {  // free the unit, then claim its place (units may leave in any order)
-            asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(u.fill + p))),
-                         "r"((~e & 0x8000u) << 9)
-                         : "memory");
+            unit_free(u.fill + p, (~e & 0x8000u) << 9);
             pos = atomicAdd(&u.cur[p], F);
         }
         pos = __shfl_sync(0xffffffffu, pos, static_cast<int>(lane - c)) + c * U::CH;
