@@ -721,7 +721,7 @@ pj_status launch_scatter_t(const K* keys, int64_t n, int64_t chunk, int items, D
     const uint32_t cap32 = static_cast<uint32_t>(std::min<int64_t>(out_cap, UINT32_MAX));
     constexpr int V = sc_v<K>();
     const int lf = unit_logf<K>(P, W, SC_THREADS, V, HEAVY ? HeavyTable::BYTES + 16 : 0);
-    if (lf >= 0 && chunk <= static_cast<int64_t>(WCU_COUNT)) {
+    if (lf >= 0) {
         // 8-byte keys over 4096 partitions: two tuples a unit, and HBM takes the
         // sectors no faster than half the warps bring them (2^28 keys 2.40 ->
         // 2.16 ms); fewer partitions wait on the warps (2048: 434 -> 473 us), as

@@ -569,10 +569,13 @@ __device__ __forceinline__ void wc_finish(int P, uint32_t* buf, int cap, WcState
 //
 // The block-wide form (three barriers per round of one vector a thread)
 // waited on shared-memory latency and barriers with half the issue slots
-// idle.  A count needs no reset bound: it grows by one per tuple of the
-// chunk at most, and a chunk has fewer than 2^24 tuples.
+// idle.  The count of a unit that stays full grows with every tuple that meets
+// it, so a block barrier every WCU_EPOCH tuples, at which no unit is full,
+// keeps it within its bits (a tuple is counted twice at most: as it comes and
+// from the late list).
 constexpr int WCU_LATE = 64;  // tuples a warp keeps to place later
 constexpr uint32_t WCU_COUNT = (1u << 24) - 1u;  // count bits of a fill word; bit 24: parity
+constexpr uint32_t WCU_EPOCH = 1u << 22;         // tuples of a CTA between barriers; a multiple of a round's
 
 template <typename K>
 struct WcUnits {
@@ -985,6 +988,7 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __res
     constexpr int NV = V / VN;  // vectors per thread per round
     static_assert(V % VN == 0, "V must be whole vectors");
     constexpr int ROUND = THREADS * V;
+    static_assert(WCU_EPOCH % ROUND == 0 && 2 * WCU_EPOCH < WCU_COUNT, "a count stays within its bits");
     extern __shared__ __align__(128) uint8_t smem[];
     WcUnits<K> wc;
     wc.bind(smem, P, logF, V);
@@ -1079,6 +1083,7 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __res
             }
             if constexpr (HEAVY) wcu_place_few<K, V>(wc, n_late, w, dv, ok, out, out_cap, status);
             else wcu_place<K, V>(wc, n_late, w, dv, ok, out, out_cap, status);
+            if (((b + ROUND) & (WCU_EPOCH - 1u)) == 0) __syncthreads();
         }
         wcu_finish<K>(wc, n_late, P, static_cast<uint32_t>(W), out, out_cap, status);
     }
@@ -1306,6 +1311,7 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_tuples_kernel(const uint32
 {
     constexpr int TW = TupleTraits<K>::WORDS;
     constexpr int ROUND = THREADS * VT;
+    static_assert(WCU_EPOCH % ROUND == 0);
     extern __shared__ __align__(128) uint8_t smem[];
     WcUnits<K> wc;
     wc.bind(smem, P, logF, VT);
@@ -1339,6 +1345,7 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_tuples_kernel(const uint32
             }
             if (b + ROUND < hi) load_round(b + ROUND);
             wcu_place<K, VT>(wc, n_late, w, dv, ok, out, out_cap, status);
+            if (((b + ROUND - lo) & (WCU_EPOCH - 1u)) == 0) __syncthreads();
         }
         wcu_finish<K>(wc, n_late, P, static_cast<uint32_t>(W), out, out_cap, status);
     }
@@ -1386,7 +1393,8 @@ __global__ void __launch_bounds__(HIST_THREADS) hist_seg_kernel(const SegItem* _
 }
 
 // Write-combining scatter of the items (persistent grid; buffers sized for
-// the largest partition count of the batch, Pmax).
+// the largest partition count of the batch, Pmax; an item's SEG_CHUNK rows
+// stay below WCU_EPOCH).
 template <typename K, int THREADS, int VT>
 __global__ void __launch_bounds__(THREADS, 1) scatter_seg_kernel(const SegItem* __restrict__ items, int32_t n_items,
                                                                  int32_t Pmax, int32_t logF, int32_t W,

@@ -35,3 +35,19 @@ def test_units_change_hands_whole(dtype, bits, used):
     assert torch.equal(got[:, 0 if words == 2 else 2], hashes.view(torch.int32)[rows[real]])
     part = torch.repeat_interleave(torch.arange(P, device="cuda"), torch.diff(offsets))
     assert torch.equal(part[real], (keys[rows[real]].long() & (P - 1)))
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+def test_second_pass_item_of_more_tuples_than_a_count_holds(dtype):
+    # one first-pass partition holds every key, so one second-pass item places
+    # more tuples than the 24 bits of a unit's count could number
+    n, words = (1 << 25) + 5, 2 if dtype == np.int32 else 4
+    keys = torch.full((n,), 12345, dtype=torch.int32 if dtype == np.int32 else torch.int64, device="cuda")
+    plan = api.plan_default(n, n, np.dtype(dtype).itemsize)
+    plan.passes, plan.bits1, plan.bits2, plan.wc_tuples = 2, 10, 2, 8 // words
+    plan.table_mode, plan.table_capacity = 0, 4096
+    tuples, offsets = api.partition(keys, plan)
+    assert int((torch.diff(offsets) > 0).sum()) == 1
+    rows = tuples[: int(offsets[-1]) * words].view(-1, words)[:, -1]
+    real = rows[rows >= 0].long()
+    assert real.numel() == n and torch.equal(torch.sort(real)[0], torch.arange(n, device="cuda"))

@@ -44,3 +44,18 @@ def test_fill_words_change_by_atomics_alone():
     assert "atom.release.cta.shared.exch.b32" in text and "atom.acquire.cta.shared.add.u32" in text
     # every lane has read its sector before one of them frees the unit
     assert re.search(r"__syncwarp\(\);\s*uint32_t pos = 0;\s*if \(act && c == 0\) \{\s*unit_free\(", put)
+
+
+def test_counts_stay_within_their_bits():
+    # items of any length: a barrier every WCU_EPOCH tuples, each counted twice at most
+    text = source()
+    bits = int(re.search(r"WCU_COUNT = \(1u << (\d+)\) - 1u", text).group(1))
+    epoch = int(re.search(r"WCU_EPOCH = 1u << (\d+)", text).group(1))
+    assert epoch + 1 < bits
+    for name in ("scatter_keys_kernel", "scatter_tuples_kernel"):
+        at = text.index(f" {name}(")
+        end = text.index("wcu_finish", at)
+        assert re.search(r"WCU_EPOCH - 1u\)\) == 0\) __syncthreads\(\);", text[at:end]), name
+    with open(os.path.join(ROOT, "partitioned_join_b200", "csrc", "pj_api.cu")) as f:
+        seg = int(re.search(r"SEG_CHUNK = 1 << (\d+)", f.read()).group(1))
+    assert seg < epoch   # items of batches
