@@ -679,10 +679,9 @@ __device__ __forceinline__ uint32_t unit_take(uint32_t* fill)
 // The unit is free again, with this fill word.
 __device__ __forceinline__ void unit_free(uint32_t* fill, uint32_t word)
 {
-    uint32_t old;
-    asm volatile("atom.release.cta.shared.exch.b32 %0, [%1], %2;"
-                 : "=r"(old)
-                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(fill))), "r"(word)
+    asm volatile("{ .reg .b32 t; atom.release.cta.shared.exch.b32 t, [%0], %1; }" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(fill))),
+                 "r"(word)
                  : "memory");
 }
 
