@@ -363,9 +363,10 @@ pj_status pj_batch_check(void* workspace, pj_stream stream);
 
 /* Autotuner: times candidate configurations on this batch (where the
  * direct path ends, the direct kernel's block size and chunk, the radix
- * width of the partitioned joins, whether they run together) and returns the
- * fastest in *best (and its
- * time, optional).  SYNCHRONISES; runs the batch many times.  The workspace
+ * width of the partitioned joins, whether joins share launches), leaving
+ * alone what reaches no join of it, and returns the fastest in *best (and its
+ * time, optional): the defaults unless another beats them by more than 2 %.
+ * SYNCHRONISES; runs the batch many times.  The workspace
  * must hold pj_batch_workspace_size for direct_max_build = 0. */
 pj_status pj_batch_autotune(const pj_join_desc* descs, const pj_output* outs, int32_t n, void* workspace,
                             size_t workspace_bytes, pj_stream stream, pj_batch_config* best, float* best_ms);

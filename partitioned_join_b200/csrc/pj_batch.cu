@@ -655,57 +655,79 @@ pj_status pj_batch_autotune(const pj_join_desc* descs, const pj_output* outs, in
     pj_batch_config cur = base;
     float cur_ms = 0;
     pj_status s = time_cfg(cur, 3, &cur_ms);
+    // Knobs that reach no join of the batch are left alone: every choice
+    // between them would be one by noise.
     // 1. where the direct path ends (whole batch timed)
-    const int limits[] = {0, 4096, 8192, 16384, 24576, DIRECT_MAX_BUILD};
-    for (int lim : limits) {
-        if (s != PJ_OK) break;
-        pj_batch_config c = cur;
-        c.direct_max_build = lim;
-        float t = 0;
-        const pj_status r = time_cfg(c, 3, &t);
-        if (r == PJ_OK && t < cur_ms) {
-            cur = c;
-            cur_ms = t;
+    auto tune_limit = [&]() {
+        pj_batch_config all = cur;
+        all.direct_max_build = DIRECT_MAX_BUILD;
+        if (split_batch(descs, n, all).direct.empty()) return;
+        for (int lim : {0, 4096, 8192, 16384, 24576, DIRECT_MAX_BUILD}) {
+            pj_batch_config c = cur;
+            c.direct_max_build = lim;
+            float t = 0;
+            if (time_cfg(c, 3, &t) == PJ_OK && t < cur_ms) {
+                cur = c;
+                cur_ms = t;
+            }
         }
-    }
+    };
     // 2. block size and chunk of the direct kernel (direct part timed)
-    if (s == PJ_OK && cur.direct_max_build > 0) {
+    auto tune_direct = [&]() {
+        if (split_batch(descs, n, cur).direct.empty()) return;
         float dbest = 0;
-        if (time_cfg(cur, 1, &dbest) == PJ_OK) {
-            for (int th : {256, 512, 1024})
-                for (int ch : {1 << 14, 1 << 16, 1 << 18}) {
-                    pj_batch_config c = cur;
-                    c.direct_threads = th;
-                    c.direct_chunk = ch;
-                    float t = 0;
-                    if (time_cfg(c, 1, &t) == PJ_OK && t < dbest) {
-                        dbest = t;
-                        cur.direct_threads = th;
-                        cur.direct_chunk = ch;
-                    }
+        if (time_cfg(cur, 1, &dbest) != PJ_OK) return;
+        for (int th : {256, 512, 1024})
+            for (int ch : {1 << 14, 1 << 16, 1 << 18}) {
+                pj_batch_config c = cur;
+                c.direct_threads = th;
+                c.direct_chunk = ch;
+                float t = 0;
+                if (time_cfg(c, 1, &t) == PJ_OK && t < dbest) {
+                    dbest = t;
+                    cur.direct_threads = th;
+                    cur.direct_chunk = ch;
                 }
-        }
-    }
-    // 3. radix width of the partitioned joins, and whether they run
-    //    together or one after another (large part timed)
+            }
+    };
+    // 3. whether joins share launches, and the radix width of the partitioned
+    //    ones (whole batch timed: joins change parts with the choice)
+    auto tune_large = [&]() {
+        for (int together : {1, 0})
+            for (int dlt : {-1, 0, 1}) {
+                if (together == cur.large_batched && dlt == cur.large_bits_delta) continue;
+                pj_batch_config c = cur;
+                c.large_bits_delta = dlt;
+                c.large_batched = together;
+                if (dlt != 0 && split_batch(descs, n, c).large.empty()) continue;
+                float t = 0;
+                if (time_cfg(c, 3, &t) == PJ_OK && t < cur_ms) {
+                    cur = c;
+                    cur_ms = t;
+                }
+            }
+    };
     if (s == PJ_OK) {
-        float lbest = 0;
-        if (time_cfg(cur, 2, &lbest) == PJ_OK) {
-            for (int together : {1, 0})
-                for (int dlt : {-1, 0, 1}) {
-                    if (together == cur.large_batched && dlt == cur.large_bits_delta) continue;
-                    pj_batch_config c = cur;
-                    c.large_bits_delta = dlt;
-                    c.large_batched = together;
-                    float t = 0;
-                    if (time_cfg(c, 2, &t) == PJ_OK && t < lbest) {
-                        lbest = t;
-                        cur.large_bits_delta = dlt;
-                        cur.large_batched = together;
-                    }
-                }
+        tune_limit();
+        tune_direct();
+        s = time_cfg(cur, 3, &cur_ms);
+    }
+    if (s == PJ_OK) {
+        tune_large();
+        if (cur.large_batched != base.large_batched) {  // other joins are direct now
+            tune_limit();
+            tune_direct();
         }
     }
+    // the winner against the defaults, in turn: a gain within 2 % is noise
+    float best_cur = 1e30f, best_base = 1e30f;
+    if (s == PJ_OK && std::memcmp(&cur, &base, sizeof(base)) != 0)
+        for (int i = 0; i < 3 && s == PJ_OK; ++i) {
+            float t = 0;
+            if ((s = time_cfg(base, 3, &t)) == PJ_OK) best_base = std::min(best_base, t);
+            if (s == PJ_OK && (s = time_cfg(cur, 3, &t)) == PJ_OK) best_cur = std::min(best_cur, t);
+        }
+    if (s == PJ_OK && !(best_cur < 0.98f * best_base)) cur = base;
     if (s == PJ_OK) {
         s = time_cfg(cur, 3, &cur_ms);
         *best = cur;
