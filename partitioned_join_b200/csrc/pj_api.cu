@@ -947,6 +947,43 @@ bool planner_made(const pj_join_desc* d, const pj_plan* p)
     return pj_plan_default(d, &q) == PJ_OK && std::memcmp(p, &q, sizeof(q)) == 0;
 }
 
+// Launches a kernel that waits for the one before it in the stream by itself
+// (griddepcontrol.wait, before it touches memory), so its blocks are in place
+// when that one ends: 2 to 4 us off a chain of five small kernels.
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kern)(P...), unsigned grid, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(GT_THREADS);
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+// Words of the list of long ranges' probe rows (GtLong), at most.
+int64_t long_words(int64_t n_probe) { return (n_probe + 32 * GT_U - 1) / (32 * GT_U); }
+
+// GtLong of a join: as many bits for the rounds as the words leave, and slices
+// so large that the rounds of any keys fit them (one step up to 2^29 x 2^22 rows).
+GtLong long_ranges(int64_t n_build, int64_t n_probe, int key_bytes, void* cursor, void* list)
+{
+    GtLong g;
+    g.cursor = static_cast<unsigned long long*>(cursor);
+    g.list = static_cast<unsigned long long*>(list);
+    const int64_t words = long_words(n_probe);
+    g.walk = n_probe < GT_WALK_PROBE ? GT_LONG : key_bytes == 4 ? GT_WALK_32 : GT_WALK_64;
+    g.round_bits = 63 - ilog2_floor(words);
+    for (g.slice = GT_SLICE;; g.slice *= 2) {
+        const int64_t slices = n_probe * ((n_build + g.slice - 1) / g.slice);  // < 2^46
+        if (words + slices / GT_ROUND < (int64_t(1) << std::min(g.round_bits, 62))) return g;
+    }
+}
+
 // The global table lives in the bytes that the partitioned layout has
 // anyway, so no workspace grows; a join whose table does not fit them
 // (many more build than probe rows) is partitioned.
@@ -972,9 +1009,12 @@ GlobalPlan global_plan(const pj_join_desc* d, const pj_plan* p, const Layout& L)
         g.use = slots * static_cast<int64_t>(g.nb) >= n + n / 2 + 8;
         return g;
     }
+    // The list of the probe rows with long ranges follows the counts in their
+    // place; it is larger only for 32 probe rows a build row, whose layout has
+    // the room many times over.
     g.nb = static_cast<uint32_t>(std::max<int64_t>(8, n));
     g.zeroed = align_up(o + 4 * static_cast<size_t>(g.nb), 256);
-    g.range = g.zeroed;
+    g.range = std::max(g.zeroed, align_up(o + 8 * static_cast<size_t>(long_words(d->n_probe)), 256));
     g.entries = align_up(g.range + 8 * static_cast<size_t>(g.nb), 256);
     g.use = g.entries + 8 * static_cast<size_t>(n) <= L.total;
     return g;
@@ -992,7 +1032,8 @@ pj_status run_global(const pj_join_desc* d, const GlobalPlan& g, const Layout& L
     auto* cnt = reinterpret_cast<unsigned long long*>(count);
     const GlobalOut o{out_b, out_p, capacity, cnt, status};
     for (int i = PJ_STAGE_BUILD_HIST; i <= PJ_STAGE_BUILD_SCATTER; ++i) E.mark(i, st);
-    PJ_CUDA(cudaMemsetAsync(ws, 0, g.zeroed, st));
+    const bool small = !d->unique_build_keys && d->n_build <= GT_GROUP;
+    if (!small) PJ_CUDA(cudaMemsetAsync(ws, 0, g.zeroed, st));
     if (d->unique_build_keys) {
         auto* table = reinterpret_cast<uint32_t*>(ws + g.table);
         gt_build_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, table, g.nb, cnt, status);
@@ -1008,17 +1049,27 @@ pj_status run_global(const pj_join_desc* d, const GlobalPlan& g, const Layout& L
         auto* counts = reinterpret_cast<uint32_t*>(ws + g.table);
         auto* range = reinterpret_cast<uint2*>(ws + g.range);
         auto* entries = reinterpret_cast<uint2*>(ws + g.entries);
-        gt_count_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, counts, g.nb, cnt);
-        PJ_CUDA(cudaGetLastError());
-        // (the counter block's words double as the 64-bit entry cursor)
+        // (the counter block's words double as 64-bit cursors: entries, and GtLong's)
         auto* cursor = reinterpret_cast<unsigned long long*>(ws + L.counters);
-        gt_alloc_kernel<<<(g.nb + GT_THREADS * GT_ALLOC - 1) / (GT_THREADS * GT_ALLOC), GT_THREADS, 0, st>>>(
-            counts, g.nb, range, cursor);
-        PJ_CUDA(cudaGetLastError());
-        gt_place_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, range, g.nb, entries);
+        if (small) {
+            gt_group_kernel<K><<<1, GT_GROUP_THREADS, 0, st>>>(bk, nb, g.nb, reinterpret_cast<uint32_t*>(ws),
+                                                               static_cast<int>(L.counters / 4) + 8, range, entries, cnt);
+        } else {
+            gt_count_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, counts, g.nb, cnt);
+            PJ_CUDA(cudaGetLastError());
+            PJ_CUDA(launch_after(gt_alloc_kernel, (g.nb + GT_THREADS * GT_ALLOC - 1) / (GT_THREADS * GT_ALLOC), st, counts,
+                                 g.nb, range, cursor));
+            PJ_CUDA(launch_after(gt_place_kernel<K>, bgrid, st, bk, nb, range, g.nb, entries));
+        }
         PJ_CUDA(cudaGetLastError());
         for (int i = PJ_STAGE_BUILD_PASS2; i <= PJ_STAGE_JOIN; ++i) E.mark(i, st);
-        gt_probe_multi_kernel<K><<<pgrid, GT_THREADS, 0, st>>>(pk, np, bk, range, g.nb, entries, o);
+        // (the list takes the counts' place: the ranges hold them by now)
+        const GtLong later = long_ranges(d->n_build, d->n_probe, d->key_bytes, cursor + 1, counts);
+        PJ_CUDA(launch_after(gt_probe_multi_kernel<K>, pgrid, st, pk, np, bk, range, g.nb, entries, later, o));
+        if (nb > GT_LONG) {
+            PJ_CUDA(launch_after(gt_probe_long_kernel<K>, static_cast<unsigned>(sm_count()) * GT_LONG_CTAS, st, pk, np, bk,
+                                 range, g.nb, entries, later, o));
+        }
     }
     PJ_CUDA(cudaGetLastError());
     return PJ_OK;

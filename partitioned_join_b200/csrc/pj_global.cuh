@@ -20,7 +20,8 @@
 //
 // Repeated build keys: rows grouped by bucket (count, allocate, place),
 // 8-byte entries {murmur(key), row} and each bucket's range; a lookup walks
-// its bucket, long ones with the whole warp.
+// its bucket.  Long buckets are left to a second launch, which cuts them into
+// slices over the whole GPU, whatever probe rows meet them.
 //
 // Reference counterpart: hash_join (hash_join_kernels.cuh:24-200), which
 // builds such a table per partition in shared memory.
@@ -38,7 +39,20 @@ constexpr int GT_U = 2;                     // probe rows of a thread in flight 
 constexpr int GT_TILE = GT_THREADS * GT_U;  // probe rows of one step of a CTA
 constexpr int GT_STEPS = 4;                 // steps of a CTA (one where the probe side does not fill the GPU)
 constexpr uint32_t GT_MAX_BUCKETS = 1u << 13;  // buckets an insert or a lookup tries
-constexpr uint32_t GT_LONG = 32;            // repeated keys: ranges beyond this are walked by the warp
+constexpr uint32_t GT_LONG = 32;            // repeated keys: longer ranges are walked by the warp or cut into slices
+constexpr int GT_SLICE_U = 2;               // entries of a slice's step in flight a lane
+constexpr uint32_t GT_SLICE = 32 * GT_SLICE_U;  // entries of a slice's step
+constexpr int GT_SLICES = 4;                // slices of a warp in flight together
+constexpr uint32_t GT_ROUND = GT_THREADS / 32 * GT_SLICES;  // slices of a CTA's round
+// From GT_WALK_PROBE probe rows on, whose tiles fill the GPU, the finder's warp
+// walks ranges of up to GT_WALK entries: 2^20 4-byte probe rows of ranges of
+// 256 take 660 us walked and 815 cut, 2^18 rows 245 and 238.  With 8-byte keys a
+// walk waits for a build key at every step (2400 us and 1536), but where few
+// rows of a warp meet a short range, a cut spends a whole round on them (2^21
+// rows, runs of 24 rows a key: 1354 us walked, 1535 cut; 96 rows: 1844 and 1951).
+constexpr int64_t GT_WALK_PROBE = int64_t(1) << 19;
+constexpr uint32_t GT_WALK_32 = 1024, GT_WALK_64 = 256;
+constexpr unsigned GT_LONG_CTAS = 4;        // CTAs per SM of the launch for them
 constexpr int GT_ROW_BITS = 22;             // 8-byte keys: row bits of a slot
 constexpr int64_t GT_MAX_BUILD = int64_t(1) << GT_ROW_BITS;  // build rows of a table
 constexpr int GT_STAGE = 2048;              // repeated keys: pairs a CTA stages for whole-run stores
@@ -401,6 +415,23 @@ __global__ void __launch_bounds__(GT_THREADS, STEPS == 1 ? 2048 / GT_THREADS : 1
                                 J->nb, o, it.row0);
 }
 
+// A kernel of the chain below: the next one may be put in place, and this one
+// goes on when the one before has ended and its writes are visible.  (What
+// that one wrote is read by plain loads: a non-coherent load wants memory that
+// nobody writes while its kernel is there, and it may be there by then.)
+__device__ __forceinline__ void gt_wait_before()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__device__ __forceinline__ uint2 gt_load(const uint2* p)
+{
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
 // ---- repeated build keys ---------------------------------------------------
 
 template <typename K>
@@ -408,6 +439,7 @@ __global__ void __launch_bounds__(GT_THREADS) gt_count_kernel(const K* __restric
                                                               uint32_t* counts, uint32_t nb,
                                                               unsigned long long* count)
 {
+    gt_wait_before();
     const uint32_t i = blockIdx.x * GT_THREADS + threadIdx.x;
     if (i == 0) *count = 0;
     if (i < n) atomicAdd(&counts[gt_bucket(hash_key(keys[i]), nb)], 1u);
@@ -417,10 +449,11 @@ __global__ void __launch_bounds__(GT_THREADS) gt_count_kernel(const K* __restric
 // CTA lie one after another, the CTAs in whatever order they come (one
 // atomic each instead of a scan over all of them).
 constexpr int GT_ALLOC = 8;  // buckets per thread
-static __global__ void __launch_bounds__(GT_THREADS) gt_alloc_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
-                                                              uint2* __restrict__ range, unsigned long long* cursor)
+static __global__ void __launch_bounds__(GT_THREADS) gt_alloc_kernel(const uint32_t* counts, uint32_t nb,
+                                                              uint2* range, unsigned long long* cursor)
 {
     __shared__ unsigned long long s_warp[GT_THREADS / 32 + 2];
+    gt_wait_before();
     const uint32_t b0 = (blockIdx.x * GT_THREADS + threadIdx.x) * GT_ALLOC;
     uint32_t c[GT_ALLOC], sum = 0;
 #pragma unroll
@@ -441,10 +474,89 @@ template <typename K>
 __global__ void __launch_bounds__(GT_THREADS) gt_place_kernel(const K* __restrict__ keys, uint32_t n, uint2* range,
                                                               uint32_t nb, uint2* __restrict__ entries)
 {
+    gt_wait_before();
     const uint32_t i = blockIdx.x * GT_THREADS + threadIdx.x;
     if (i >= n) return;
     const uint32_t h = hash_key(keys[i]);
     entries[atomicAdd(&range[gt_bucket(h, nb)].y, 1u)] = make_uint2(h, i);
+}
+
+// Count, allocate and place by one CTA, the buckets' counts in shared memory,
+// and what a memset would clear (head): four launches' work in one for builds
+// of up to GT_GROUP rows, whose joins wait for launches.
+constexpr int GT_GROUP_THREADS = 1024;
+constexpr int64_t GT_GROUP = 4096;
+template <typename K>
+__global__ void __launch_bounds__(GT_GROUP_THREADS) gt_group_kernel(const K* __restrict__ keys, uint32_t n,
+                                                                    uint32_t nb, uint32_t* head, int head_words,
+                                                                    uint2* __restrict__ range,
+                                                                    uint2* __restrict__ entries,
+                                                                    unsigned long long* count)
+{
+    constexpr int U = 4;  // rows of a thread in flight
+    constexpr uint32_t T = GT_GROUP_THREADS;
+    __shared__ uint32_t s_at[GT_GROUP];  // counts, then places
+    __shared__ uint32_t s_warp[32];
+    gt_wait_before();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint32_t b = threadIdx.x; b < nb; b += T) s_at[b] = 0u;
+    for (int i = threadIdx.x; i < head_words; i += T) head[i] = 0u;
+    if (threadIdx.x == 0) *count = 0;
+    auto each = [&](auto&& f) {
+        for (uint32_t i0 = threadIdx.x; i0 < n; i0 += U * T) {
+            K k[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) k[u] = i0 + u * T < n ? keys[i0 + u * T] : K(0);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + u * T < n) f(i0 + u * T, hash_key(k[u]));
+        }
+    };
+    __syncthreads();
+    each([&](uint32_t, uint32_t h) { atomicAdd(&s_at[gt_bucket(h, nb)], 1u); });
+    __syncthreads();
+    // (an odd run: the lanes walk 32 banks)
+    const uint32_t run = ((nb + T - 1) / T) | 1u, b0 = threadIdx.x * run, b1 = min(b0 + run, nb);
+    uint32_t sum = 0;
+    for (uint32_t b = b0; b < b1; ++b) sum += s_at[b];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - sum + __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[lane] : 0u);
+    for (uint32_t b = b0; b < b1; ++b) {
+        const uint32_t c = s_at[b];
+        s_at[b] = at;
+        range[b] = make_uint2(at, at + c);
+        at += c;
+    }
+    __syncthreads();
+    each([&](uint32_t i, uint32_t h) { entries[atomicAdd(&s_at[gt_bucket(h, nb)], 1u)] = make_uint2(h, i); });
+}
+
+// Probe rows that meet a long range, for gt_probe_long_kernel: one word per
+// warp of gt_probe_multi_kernel (64 probe rows) that has such rows, and a
+// cursor over words and rounds of GT_ROUND slices.
+struct GtLong {
+    unsigned long long* cursor;  // words << round_bits | rounds
+    unsigned long long* list;    // unit << round_bits | rounds of the words before it
+    int32_t round_bits;
+    uint32_t slice;              // entries of a slice: a multiple of GT_SLICE
+    uint32_t walk;               // longer ranges are cut
+    __device__ __forceinline__ uint32_t slices(uint32_t entries) const
+    {
+        return entries > walk ? (entries + slice - 1) / slice : 0u;
+    }
+};
+
+template <typename K>
+__device__ __forceinline__ bool gt_equal(const uint2& e, uint32_t h, K key, const K* __restrict__ bkeys)
+{
+    return e.x == h && (sizeof(K) == 4 || bkeys[e.y] == key);
 }
 
 // Probe of the grouped rows: a counting walk, then a writing walk at the
@@ -455,42 +567,51 @@ __global__ void __launch_bounds__(GT_THREADS) gt_place_kernel(const K* __restric
 template <typename K>
 __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __restrict__ pkeys, uint32_t n,
                                                                     const K* __restrict__ bkeys,
-                                                                    const uint2* __restrict__ range, uint32_t nb,
-                                                                    const uint2* __restrict__ entries, GlobalOut o)
+                                                                    const uint2* range, uint32_t nb,
+                                                                    const uint2* entries, GtLong later,
+                                                                    GlobalOut o)
 {
     __shared__ unsigned long long s_warp[GT_THREADS / 32 + 2];
     __shared__ uint2 s_pair[GT_STAGE];
+    gt_wait_before();
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t row0 = blockIdx.x * GT_TILE + threadIdx.x * GT_U;
     K k[GT_U];
     uint32_t h[GT_U], lo[GT_U], hi[GT_U], c[GT_U];
     gt_load_pair<K>(pkeys, true, n, row0, k);
+    uint32_t slices = 0;
 #pragma unroll
     for (int u = 0; u < GT_U; ++u) {
         h[u] = hash_key(k[u]);
         uint2 r = make_uint2(0u, 0u);
-        if (row0 + u < n) r = __ldg(range + gt_bucket(h[u], nb));
+        if (row0 + u < n) r = gt_load(range + gt_bucket(h[u], nb));
+        const uint32_t s = later.slices(r.y - r.x);
+        slices += s;
         lo[u] = r.x;
-        hi[u] = r.y;
+        hi[u] = s ? r.x : r.y;
     }
-    auto equal = [&](const uint2& e, uint32_t hh, K kk) -> bool {
-        return e.x == hh && (sizeof(K) == 4 || bkeys[e.y] == kk);
-    };
+    slices = __reduce_add_sync(0xffffffffu, slices);
+    if (slices && lane == 0) {
+        const unsigned long long rounds = (slices + GT_ROUND - 1) / GT_ROUND;
+        const unsigned long long at = atomicAdd(later.cursor, (1ull << later.round_bits) + rounds);
+        const unsigned long long unit = row0 / (32 * GT_U);
+        later.list[at >> later.round_bits] = (unit << later.round_bits) | (at & ((1ull << later.round_bits) - 1ull));
+    }
     unsigned long long mine = 0;
 #pragma unroll
     for (int u = 0; u < GT_U; ++u) {
         c[u] = 0;
         const bool is_long = hi[u] - lo[u] > GT_LONG;
         if (!is_long)
-            for (uint32_t i = lo[u]; i < hi[u]; ++i) c[u] += equal(__ldg(entries + i), h[u], k[u]) ? 1u : 0u;
+            for (uint32_t i = lo[u]; i < hi[u]; ++i) c[u] += gt_equal<K>(gt_load(entries + i), h[u], k[u], bkeys) ? 1u : 0u;
         for (uint32_t todo = __ballot_sync(0xffffffffu, is_long); todo; todo &= todo - 1u) {
             const int owner = __ffs(todo) - 1;
             const uint32_t a = __shfl_sync(0xffffffffu, lo[u], owner), z = __shfl_sync(0xffffffffu, hi[u], owner);
             const uint32_t hh = __shfl_sync(0xffffffffu, h[u], owner);
             const K kk = __shfl_sync(0xffffffffu, k[u], owner);
             uint32_t found = 0;
-            for (uint32_t i = a + lane; i < z; i += 32) found += equal(__ldg(entries + i), hh, kk) ? 1u : 0u;
+            for (uint32_t i = a + lane; i < z; i += 32) found += gt_equal<K>(gt_load(entries + i), hh, kk, bkeys) ? 1u : 0u;
             found = __reduce_add_sync(0xffffffffu, found);
             if (lane == owner) c[u] = found;
         }
@@ -509,8 +630,8 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
         const bool is_long = hi[u] - lo[u] > GT_LONG;
         if (!is_long && c[u] > 0)
             for (uint32_t i = lo[u]; i < hi[u]; ++i) {
-                const uint2 e = __ldg(entries + i);
-                if (equal(e, h[u], k[u])) put(pos++, e.y, row0 + u);
+                const uint2 e = gt_load(entries + i);
+                if (gt_equal<K>(e, h[u], k[u], bkeys)) put(pos++, e.y, row0 + u);
             }
         for (uint32_t todo = __ballot_sync(0xffffffffu, is_long && c[u] > 0); todo; todo &= todo - 1u) {
             const int owner = __ffs(todo) - 1;
@@ -522,8 +643,8 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
             for (uint32_t i0 = a; i0 < z; i0 += 32) {
                 const uint32_t i = i0 + lane;
                 uint2 e = make_uint2(0u, 0u);
-                if (i < z) e = __ldg(entries + i);
-                const bool hit = i < z && equal(e, hh, kk);
+                if (i < z) e = gt_load(entries + i);
+                const bool hit = i < z && gt_equal<K>(e, hh, kk, bkeys);
                 const uint32_t bal = __ballot_sync(0xffffffffu, hit);
                 if (hit) put(at + __popc(bal & lt), e.y, r);
                 at += __popc(bal);
@@ -536,6 +657,130 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
     for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(all); i += GT_THREADS) {
         const uint2 p = s_pair[i];
         gt_store_pair(o, first + i, static_cast<int32_t>(p.x), p.y);
+    }
+}
+
+// The probe rows that gt_probe_multi_kernel left: the rounds of all words, in
+// equal shares over the CTAs.  A warp takes four (probe row, slice of its
+// range) a round; their entries stay in registers from the comparison to the
+// store, so a range is walked once, and the pairs of a round leave in whole
+// runs at a position reserved by one atomic.  (Walked by one warp a row,
+// 64 probe rows of a key with 2^20 build rows took 1.27 s.)
+template <typename K>
+__global__ void __launch_bounds__(GT_THREADS) gt_probe_long_kernel(const K* __restrict__ pkeys, uint32_t n,
+                                                                   const K* __restrict__ bkeys,
+                                                                   const uint2* range, uint32_t nb,
+                                                                   const uint2* entries, GtLong later,
+                                                                   GlobalOut o)
+{
+    constexpr uint32_t ROWS = 32 * GT_U;  // probe rows of a word
+    static_assert(ROWS == 64, "two rows a lane");
+    constexpr int NW = GT_THREADS / 32;
+    __shared__ unsigned long long s_warp[2][NW + 2];
+    __shared__ K s_key[ROWS];
+    __shared__ uint32_t s_hash[ROWS], s_lo[ROWS], s_hi[ROWS], s_first[ROWS];  // s_first: slices of the rows before
+    __shared__ uint32_t s_half;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    gt_wait_before();
+    const unsigned long long mask = (1ull << later.round_bits) - 1ull, all = *later.cursor;
+    const unsigned long long rounds = all & mask;
+    const uint32_t words = static_cast<uint32_t>(all >> later.round_bits);
+    unsigned long long r = rounds / gridDim.x * blockIdx.x + min(rounds % gridDim.x, static_cast<unsigned long long>(blockIdx.x));
+    const unsigned long long end = r + rounds / gridDim.x + (blockIdx.x < rounds % gridDim.x ? 1 : 0);
+    if (r == end) return;
+    // the word of the first round: the last one that starts at it or before
+    uint32_t w = 0;
+    for (uint32_t count = words; count > 1u;) {
+        const uint32_t half = count / 2u;
+        if ((later.list[w + half] & mask) <= r) {
+            w += half;
+            count -= half;
+        } else {
+            count = half;
+        }
+    }
+    int buffer = 0;
+    while (r < end) {
+        const unsigned long long word = later.list[w], word_first = word & mask;
+        const unsigned long long word_end = w + 1u < words ? later.list[w + 1u] & mask : rounds;
+        const uint32_t row0 = static_cast<uint32_t>(word >> later.round_bits) * ROWS;
+        __syncthreads();  // (every warp has left the word before)
+        uint32_t mine = 0, incl = 0;
+        if (threadIdx.x < ROWS) {
+            const uint32_t row = row0 + threadIdx.x;
+            K key = 0;
+            uint32_t h = 0;
+            uint2 x = make_uint2(0u, 0u);
+            if (row < n) {
+                key = pkeys[row];
+                h = hash_key(key);
+                x = gt_load(range + gt_bucket(h, nb));
+            }
+            incl = mine = later.slices(x.y - x.x);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += y;
+            }
+            if (threadIdx.x == 31) s_half = incl;
+            s_key[threadIdx.x] = key;
+            s_hash[threadIdx.x] = h;
+            s_lo[threadIdx.x] = x.x;
+            s_hi[threadIdx.x] = x.y;
+        }
+        __syncthreads();
+        if (threadIdx.x < ROWS) s_first[threadIdx.x] = incl - mine + (warp > 0 ? s_half : 0u);
+        __syncthreads();
+        const unsigned long long stop = word_end < end ? word_end : end;
+        for (; r < stop; ++r) {
+            const uint32_t first = (static_cast<uint32_t>(r - word_first) * NW + warp) * GT_SLICES;
+            int row[GT_SLICES];
+            uint32_t lo[GT_SLICES], hi[GT_SLICES];
+#pragma unroll
+            for (int t = 0; t < GT_SLICES; ++t) {
+                // the last row whose slices start at the slice or before (rows without slices start where the next does)
+                const int j = __popc(__ballot_sync(0xffffffffu, s_first[lane] <= first + t)) +
+                              __popc(__ballot_sync(0xffffffffu, s_first[lane + 32] <= first + t)) - 1;
+                const uint32_t part = first + t - s_first[j], from = s_lo[j], to = s_hi[j];
+                row[t] = j;
+                lo[t] = from + part * later.slice;
+                // (past the word's last slice: nothing)
+                hi[t] = part < later.slices(to - from) ? min(lo[t] + later.slice, to) : 0u;
+            }
+            for (uint32_t step = 0; step < later.slice; step += GT_SLICE, buffer ^= 1) {
+                uint2 e[GT_SLICES][GT_SLICE_U];
+#pragma unroll
+                for (int t = 0; t < GT_SLICES; ++t)
+#pragma unroll
+                    for (int v = 0; v < GT_SLICE_U; ++v) {
+                        const uint32_t i = lo[t] + step + v * 32 + lane;
+                        e[t][v] = i < hi[t] ? gt_load(entries + i) : make_uint2(~s_hash[row[t]], 0u);
+                    }
+                uint32_t off[GT_SLICES][GT_SLICE_U], hits = 0, total = 0;
+#pragma unroll
+                for (int t = 0; t < GT_SLICES; ++t)
+#pragma unroll
+                    for (int v = 0; v < GT_SLICE_U; ++v) {
+                        const bool hit = gt_equal<K>(e[t][v], s_hash[row[t]], s_key[row[t]], bkeys);
+                        const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+                        off[t][v] = total + __popc(bal & lt);
+                        total += __popc(bal);
+                        hits |= hit ? 1u << (t * GT_SLICE_U + v) : 0u;
+                    }
+                // lane 31 speaks for the warp: its position is the warp's base
+                const unsigned long long at = gt_reserve(lane == 31 ? total : 0u, s_warp[buffer], o.count);
+                const unsigned long long base = __shfl_sync(0xffffffffu, at, 31);
+                if (o.out_build == nullptr) continue;
+#pragma unroll
+                for (int t = 0; t < GT_SLICES; ++t)
+#pragma unroll
+                    for (int v = 0; v < GT_SLICE_U; ++v)
+                        if (hits >> (t * GT_SLICE_U + v) & 1u)
+                            gt_store_pair(o, base + off[t][v], static_cast<int32_t>(e[t][v].y), row0 + row[t]);
+            }
+        }
+        ++w;
     }
 }
 
