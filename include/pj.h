@@ -120,9 +120,10 @@ enum {
 
 /* pj_plan.flags: a planner made this plan for the join's sizes (pj_plan_exact,
  * pj_plan_learned), so a join whose build side's hash table stays in L2 may
- * skip the partitions; the pairs are those of any plan.  A default plan that
- * the caller did not change counts as such without the flag; a plan
- * without it runs as written. */
+ * skip the partitions; the pairs are those of any plan.  The bits above this
+ * one hold the planner's checksum of the other fields: a plan that the caller
+ * changes afterwards runs as written, as does one without the flag -- except
+ * the unchanged default plan, which counts as a planner's. */
 #define PJ_PLAN_FLAG_AUTO 1
 
 /* Execution plan.  pj_plan_default() fills it from the sizes alone,
@@ -147,7 +148,7 @@ typedef struct pj_plan {
     int32_t scatter_ctas_per_sm;/* scatter chunks per SM */
     int32_t hist_split;         /* histogram CTAs per scatter chunk */
     float max_fill;             /* OPEN: target fill (the reference's HASH_TABLE_OCC = 0.5) */
-    int32_t flags;              /* PJ_PLAN_FLAG_* */
+    int32_t flags;              /* 0, or the planner's mark (PJ_PLAN_FLAG_AUTO) */
     int32_t n_heavy;            /* heavy probe keys below (0: no heavy-key path) */
     int32_t heavy_reserved;     /* 0 */
     int64_t heavy_keys[PJ_MAX_HEAVY]; /* probe keys matched outside the partitions, by a

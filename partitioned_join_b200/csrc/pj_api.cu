@@ -2,6 +2,7 @@
 // layout and the stage sequence (the reference's main.cu:762-892).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -938,11 +939,30 @@ struct GlobalPlan {
     size_t range = 0, entries = 0;  // repeated keys
 };
 
+// PJ_PLAN_FLAG_AUTO and, above it, a checksum (FNV-1a) of the fields that say
+// what to run: whatever a caller changes after the planner, the mark is void.
+int32_t auto_flags(const pj_plan* p)
+{
+    static_assert(offsetof(pj_plan, heavy_keys) == 64, "the scalar fields");
+    uint64_t h = 0xcbf29ce484222325ull;
+    auto add = [&](uint64_t x) { h = (h ^ x) * 0x100000001b3ull; };
+    int32_t head[16];
+    std::memcpy(head, p, sizeof(head));
+    head[offsetof(pj_plan, flags) / 4] = 0;
+    for (int32_t x : head) add(static_cast<uint32_t>(x));
+    for (int i = 0; i < std::min(p->n_heavy, PJ_MAX_HEAVY); ++i) {
+        const uint64_t k = static_cast<uint64_t>(p->heavy_keys[i]);
+        add(k & 0xffffffffu);
+        add(k >> 32);
+    }
+    return static_cast<int32_t>(static_cast<uint32_t>(h >> 32) | PJ_PLAN_FLAG_AUTO);
+}
+
 // Whether a planner's schedule (not one a caller wrote) is asked for: the
-// default plan unchanged, or PJ_PLAN_FLAG_AUTO.
+// default plan unchanged, or PJ_PLAN_FLAG_AUTO with its checksum.
 bool planner_made(const pj_join_desc* d, const pj_plan* p)
 {
-    if (p->flags & PJ_PLAN_FLAG_AUTO) return true;
+    if ((p->flags & PJ_PLAN_FLAG_AUTO) && p->flags == auto_flags(p)) return true;
     pj_plan q;
     return pj_plan_default(d, &q) == PJ_OK && std::memcmp(p, &q, sizeof(q)) == 0;
 }
@@ -1721,7 +1741,7 @@ pj_status pj_plan_exact(const pj_join_desc* d, void* ws, size_t ws_bytes, pj_pla
     // Hash splits cannot separate repeated keys: a partition beyond what
     // 2^MAX_SPLIT_LOG2 tables hold (duplicates) takes the position split.
     if (mx_plan > cap * (int64_t(1) << MAX_SPLIT_LOG2) / 2) p.split_mode = PJ_SPLIT_POSITION;
-    if (d->n_build <= GLOBAL_MAX_BUILD) p.flags = PJ_PLAN_FLAG_AUTO;
+    if (d->n_build <= GLOBAL_MAX_BUILD) p.flags = auto_flags(&p);
     *plan = p;
     return PJ_OK;
 }
@@ -1871,7 +1891,7 @@ pj_status pj_plan_learned(const pj_join_desc* d, const float* params, void* ws, 
             const double m = static_cast<double>(d->n_build) / static_cast<double>(int64_t(1) << plan->bits1);
             if (d->n_build <= GLOBAL_MAX_BUILD &&
                 (plan->table_mode != PJ_TABLE_COMPACT || m + 4.0 * std::sqrt(m) <= static_cast<double>(COMPACT_RANGE)))
-                plan->flags = PJ_PLAN_FLAG_AUTO;
+                plan->flags = auto_flags(plan);
             return PJ_OK;
         }
     }
