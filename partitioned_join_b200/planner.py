@@ -198,6 +198,21 @@ def _time_join(desc, plan, ws, nb, out, reps=2) -> (float, int):
     return best, status
 
 
+# Joins of up to this many build rows take one hash table in L2 under any
+# planner's plan (pj_plan_exact, pj_plan_learned): there is no schedule to choose.
+TABLE_LOG2_BUILD = 22
+
+
+def sweep_range(min_log2_build: float, max_log2_build: float):
+    """The build sizes (log2) of a sweep that compares schedules: those above
+    2^22 rows.  Below, the exact plan would time the table and the candidates
+    the partitions that no planner's plan takes there."""
+    lo = max(float(min_log2_build), math.log2((1 << TABLE_LOG2_BUILD) + 1) + 1e-6)
+    if max_log2_build <= lo:
+        raise ValueError(f"a sweep needs build sides above 2^{TABLE_LOG2_BUILD} rows")
+    return lo, float(max_log2_build)
+
+
 def sweep_workload(rng: np.random.Generator, max_log2_build=28, max_log2_probe=29, device="cuda",
                    min_log2_build=18):
     """One seeded workload of the planner sweep: build rows log-uniform in
@@ -220,7 +235,8 @@ def sweep_workload(rng: np.random.Generator, max_log2_build=28, max_log2_probe=2
 
 
 def measure(build, probe):
-    """Features and the time of every candidate and of the exact plan."""
+    """Features and the time of every candidate and of the exact plan (build
+    sides above 2^22 rows: sweep_range)."""
     feat, heavy = features(build, probe)
     d = api.make_desc(build, probe, True)
     cands = [candidate(build, probe, c, heavy) for c in range(_lib.PLAN_CANDIDATES)]
@@ -293,7 +309,8 @@ def main():
     ap.add_argument("--held-out", type=float, default=0.25)
     ap.add_argument("--steps", type=int, default=3000)
     ap.add_argument("--seed", type=int, default=11)
-    ap.add_argument("--min-log2-build", type=int, default=18)
+    ap.add_argument("--min-log2-build", type=int, default=TABLE_LOG2_BUILD,
+                    help="smallest build side of the sweep (at least 2^22 rows)")
     ap.add_argument("--max-log2-build", type=int, default=28)
     ap.add_argument("--max-log2-probe", type=int, default=29)
     ap.add_argument("--out", default=WEIGHTS)
@@ -304,7 +321,9 @@ def main():
     rng = np.random.default_rng(a.seed)
     F, T, FAIL, TEX, META = [], [], [], [], []
     t0 = time.time()
-    if a.from_data:
+    if not a.from_data:
+        lo, hi = sweep_range(a.min_log2_build, a.max_log2_build)
+    else:
         for path in a.from_data.split(","):
             z = np.load(path)
             F += list(z["features"])
@@ -317,7 +336,7 @@ def main():
         F, T, FAIL, TEX, META = ([x[i] for i in order] for x in (F, T, FAIL, TEX, META))
         a.workloads = len(F)
     for i in range(0 if a.from_data else a.workloads):
-        b, p, meta = sweep_workload(rng, a.max_log2_build, a.max_log2_probe, min_log2_build=a.min_log2_build)
+        b, p, meta = sweep_workload(rng, hi, a.max_log2_probe, min_log2_build=lo)
         f, t, fl, te = measure(b, p)
         F.append(f), T.append(t), FAIL.append(fl), TEX.append(te), META.append(meta)
         del b, p
