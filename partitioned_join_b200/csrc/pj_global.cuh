@@ -40,6 +40,7 @@ constexpr int GT_TILE = GT_THREADS * GT_U;  // probe rows of one step of a CTA
 constexpr int GT_STEPS = 4;                 // steps of a CTA (one where the probe side does not fill the GPU)
 constexpr uint32_t GT_MAX_BUCKETS = 1u << 13;  // buckets an insert or a lookup tries
 constexpr uint32_t GT_LONG = 32;            // repeated keys: longer ranges are walked by the warp or cut into slices
+constexpr int GT_WALK_U = 4;                // entries of a short range in flight a lane
 constexpr int GT_SLICE_U = 2;               // entries of a slice's step in flight a lane
 constexpr uint32_t GT_SLICE = 32 * GT_SLICE_U;  // entries of a slice's step
 constexpr int GT_SLICES = 4;                // slices of a warp in flight together
@@ -579,6 +580,7 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
     const uint32_t row0 = blockIdx.x * GT_TILE + threadIdx.x * GT_U;
     K k[GT_U];
     uint32_t h[GT_U], lo[GT_U], hi[GT_U], c[GT_U];
+    uint32_t hit[GT_U];  // entries of a short range that match
     gt_load_pair<K>(pkeys, true, n, row0, k);
     uint32_t slices = 0;
 #pragma unroll
@@ -603,8 +605,20 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
     for (int u = 0; u < GT_U; ++u) {
         c[u] = 0;
         const bool is_long = hi[u] - lo[u] > GT_LONG;
-        if (!is_long)
-            for (uint32_t i = lo[u]; i < hi[u]; ++i) c[u] += gt_equal<K>(gt_load(entries + i), h[u], k[u], bkeys) ? 1u : 0u;
+        hit[u] = 0;
+        if (!is_long) {
+            for (uint32_t i = lo[u]; i < hi[u]; i += GT_WALK_U) {
+                uint2 e[GT_WALK_U];
+                bool eq[GT_WALK_U];
+#pragma unroll
+                for (int v = 0; v < GT_WALK_U; ++v) e[v] = i + v < hi[u] ? gt_load(entries + i + v) : make_uint2(~h[u], 0u);
+#pragma unroll
+                for (int v = 0; v < GT_WALK_U; ++v) eq[v] = gt_equal<K>(e[v], h[u], k[u], bkeys);
+#pragma unroll
+                for (int v = 0; v < GT_WALK_U; ++v) hit[u] |= eq[v] ? 1u << (i - lo[u] + v) : 0u;
+            }
+            c[u] = __popc(hit[u]);
+        }
         for (uint32_t todo = __ballot_sync(0xffffffffu, is_long); todo; todo &= todo - 1u) {
             const int owner = __ffs(todo) - 1;
             const uint32_t a = __shfl_sync(0xffffffffu, lo[u], owner), z = __shfl_sync(0xffffffffu, hi[u], owner);
@@ -628,11 +642,7 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
 #pragma unroll
     for (int u = 0; u < GT_U; ++u) {
         const bool is_long = hi[u] - lo[u] > GT_LONG;
-        if (!is_long && c[u] > 0)
-            for (uint32_t i = lo[u]; i < hi[u]; ++i) {
-                const uint2 e = gt_load(entries + i);
-                if (gt_equal<K>(e, h[u], k[u], bkeys)) put(pos++, e.y, row0 + u);
-            }
+        for (uint32_t m = hit[u]; m; m &= m - 1u) put(pos++, gt_load(entries + lo[u] + __ffs(m) - 1).y, row0 + u);
         for (uint32_t todo = __ballot_sync(0xffffffffu, is_long && c[u] > 0); todo; todo &= todo - 1u) {
             const int owner = __ffs(todo) - 1;
             const uint32_t a = __shfl_sync(0xffffffffu, lo[u], owner), z = __shfl_sync(0xffffffffu, hi[u], owner);

@@ -33,8 +33,9 @@ def run_keys(rng, copies, runs, others, dtype):
     return b, k
 
 
-# a range is cut from 33 entries on; slices end at multiples of 256, a warp's rounds at 8 slices
-@pytest.mark.parametrize("copies", [32, 33, 255, 256, 257, 2048, 2049])
+# up to 32 entries are walked by a lane, four at a time; a range is cut from 33 entries on, into slices of 64, 32 of
+# them a round
+@pytest.mark.parametrize("copies", [1, 3, 4, 5, 31, 32, 33, 63, 64, 65, 255, 2048, 2049])
 @pytest.mark.parametrize("dtype", [np.int32, np.int64])
 @pytest.mark.parametrize("n_probe", [1, 65, 5000])
 def test_ranges_around_the_slices(copies, dtype, n_probe):
@@ -149,4 +150,33 @@ def test_a_hot_build_key_uses_the_whole_gpu(dtype):
         # every hot build row with every hot probe row once
         x = torch.unique(j.probe_row.long() * nb + j.build_row.long())
         assert x.numel() == n and int(x.max()) < hits * nb and bool((bt[(x % nb)] == -7).all())
+    assert best[0] < best[1], best
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+def test_few_rows_a_key_gain_from_the_table(dtype):
+    # 16 probe rows a build row, four build rows a key: the table is the faster route for both key widths
+    nb, n_probe = 1 << 20, 1 << 24
+    rng = np.random.default_rng(12)
+    b = (rng.permutation(nb) // 4 * 0x1003F).astype(dtype)
+    p = (rng.integers(0, 3 * nb // 8, n_probe) * 0x1003F).astype(dtype)
+    bt, pt = dev(b), dev(p)
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    best = []
+    for written in (False, True):
+        plan = api.plan_default(nb, n_probe, b.itemsize, False)
+        if written:
+            plan.hist_split = 1 if plan.hist_split != 1 else 2
+        j = api.Joiner(bt, pt, False, plan)
+        t = []
+        for _ in range(5):
+            e0.record()
+            j.launch()
+            e1.record()
+            torch.cuda.synchronize()
+            t.append(e0.elapsed_time(e1))
+        best.append(min(t))
+        br, pr = j.result()
+        assert br.numel() == 4 * int((p < nb // 4 * 0x1003F).sum()) if dtype == np.int64 else br.numel() > 0
+        assert bool((bt[br.long()] == pt[pr.long()]).all())
     assert best[0] < best[1], best
