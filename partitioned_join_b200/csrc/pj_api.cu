@@ -11,7 +11,7 @@
 
 #include <cuda_runtime.h>
 
-#include "../../include/pj.h"
+#include "/root/repo/include/pj.h"
 #include "pj_device.cuh"
 #include "pj_global.cuh"
 #include "pj_internal.h"
@@ -681,17 +681,22 @@ pj_status launch_scan(const TIn* in, int64_t m, uint32_t round_to, int64_t* out,
 
 // log2 of the tuples of a write-combining unit for P partitions: whole
 // sectors, at least W, and as large as about 128 KB over all partitions allow
-// (the fewer partitions, the more tuples of a round meet in one unit); -1
-// where units and cursors do not fit beside `extra` bytes.
+// (the fewer partitions, the more tuples of a round meet in one unit), but at
+// most a quarter of what an item of `rows` rows brings a partition: every unit is
+// cleared before the item and written part full after it (2^21 int32 keys over
+// 128 partitions 25.4 -> 21.5 us, 2^19 19.4 -> 11.2; an eighth costs 2^24
+// keys over 1024 partitions 3 us of 89); -1 where units and cursors do not fit
+// beside `extra` bytes.
 template <typename K>
-int unit_logf(int P, int W, int threads, int v, size_t extra)
+int unit_logf(int P, int W, int threads, int v, size_t extra, int64_t rows)
 {
     using U = WcUnits<K>;
     int lf = U::LOG_CH;
     while ((1 << lf) < W) ++lf;
     if (lf > U::MAX_LOGF || U::bytes(P, lf, threads, v) + extra > smem_limit()) return -1;
     while (lf < U::MAX_LOGF && (static_cast<size_t>(P) << (lf + 1)) * U::TW * 4 <= (size_t(128) << 10) &&
-           U::bytes(P, lf + 1, threads, v) + extra <= smem_limit())
+           U::bytes(P, lf + 1, threads, v) + extra <= smem_limit() &&
+           (static_cast<int64_t>(P) << (lf + 1)) * 4 <= rows)
         ++lf;
     return lf;
 }
@@ -721,7 +726,7 @@ pj_status launch_scatter_t(const K* keys, int64_t n, int64_t chunk, int items, D
     if constexpr (HEAVY) h = *hc.hs;
     const uint32_t cap32 = static_cast<uint32_t>(std::min<int64_t>(out_cap, UINT32_MAX));
     constexpr int V = sc_v<K>();
-    const int lf = unit_logf<K>(P, W, SC_THREADS, V, HEAVY ? HeavyTable::BYTES + 16 : 0);
+    const int lf = unit_logf<K>(P, W, SC_THREADS, V, HEAVY ? HeavyTable::BYTES + 16 : 0, chunk);
     if (lf >= 0) {
         // 8-byte keys over 4096 partitions: two tuples a unit, and HBM takes the
         // sectors no faster than half the warps bring them (2^28 keys 2.40 ->
@@ -869,7 +874,7 @@ pj_status launch_scatter_tuples(const uint32_t* in, const Pass2Items& it, int n_
 {
     constexpr int VT = sizeof(K) == 4 ? 4 : 2;
     auto* kern = scatter_tuples_kernel<K, SC_THREADS, VT>;
-    const int lf = unit_logf<K>(P2, W, SC_THREADS, VT, 0);
+    const int lf = unit_logf<K>(P2, W, SC_THREADS, VT, 0, INT64_MAX);
     if (lf < 0) return PJ_ERR_INVALID;
     const size_t smem = WcUnits<K>::bytes(P2, lf, SC_THREADS, VT);
     PJ_CUDA(set_smem(kern, smem));
@@ -1933,7 +1938,7 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
                                    reinterpret_cast<uint64_t*>(w + lb.o_tiles), ctr + CTR_BTILE, status, st)) != PJ_OK)
         return s;
     constexpr int VT = sizeof(K) == 4 ? 4 : 2;
-    const int lf = unit_logf<K>(lb.Pmax, lb.W, SC_THREADS, VT, 0);
+    const int lf = unit_logf<K>(lb.Pmax, lb.W, SC_THREADS, VT, 0, INT64_MAX);
     if (lf < 0) return PJ_ERR_INVALID;
     const size_t ssmem = WcUnits<K>::bytes(lb.Pmax, lf, SC_THREADS, VT);
     const uint32_t out_cap = static_cast<uint32_t>(std::min<int64_t>(lb.tuples, UINT32_MAX));
