@@ -11,7 +11,7 @@
 
 #include <cuda_runtime.h>
 
-#include "/root/repo/include/pj.h"
+#include "../../include/pj.h"
 #include "pj_device.cuh"
 #include "pj_global.cuh"
 #include "pj_internal.h"
@@ -27,12 +27,13 @@ namespace {
 // Fixed kernel configurations.
 constexpr int SC_THREADS = 1024;
 constexpr int SC_V32 = 4, SC_V64 = 2;  // keys per thread per round (one 16-byte vector)
-// Working threads of a join CTA (and one planner warp beside them).  24 warps
-// of 72 registers for 4-byte keys, 23 of 80 for 8-byte keys, whose probe spills
-// at 72 (25 warps leave one quarter of the SM seven): 2^24 x 2^26 int64 628 ->
-// 597 us, 2^27 x 2^27 int32 with 23 warps 1.09 -> 1.13 ms.
+// Working threads of a join CTA: 24 warps of up to 80 registers where a
+// partition is one range.  Over several ranges, with a planner warp beside them,
+// 24 of 72 for 4-byte keys and 23 of 80 for 8-byte keys, whose probe spills at 72
+// (25 warps leave one quarter of the SM seven): 2^27 x 2^27 int32 with 23
+// warps 1.09 -> 1.13 ms.
 template <typename K>
-constexpr int jn_threads() { return sizeof(K) == 4 ? 768 : 736; }
+constexpr int jn_threads(int ng) { return sizeof(K) == 4 || ng == 1 ? 768 : 736; }
 constexpr int JN_BLOCK_MAX = 768 + 32;
 constexpr int MAX_SPLIT_LOG2 = 6;
 constexpr int MAX_BUCKET_CAP = 65535;  // 16-bit bucket ends
@@ -769,14 +770,14 @@ pj_status launch_scatter(const K* keys, int64_t n, int64_t chunk, int items, Dig
 template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF, int NG>
 pj_status launch_join_g(const JoinArgs& a, cudaStream_t st)
 {
-    auto* kern = join_kernel<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, jn_threads<K>(), NG>;
+    auto* kern = join_kernel<K, TABLE, UNIQUE, HASH_SPLIT, SLOT_REF, jn_threads<K>(NG), NG>;
     const size_t smem = JoinSmem<K, TABLE>::bytes(a.cap, a.nb_log2);
     PJ_CUDA(set_smem(kern, smem));
     int per_sm = 0;
-    PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, jn_threads<K>() + 32, smem));
+    PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, jn_threads<K>(NG) + JOIN_PLANNERS<NG>, smem));
     per_sm = std::min(std::max(per_sm, 1), MAX_JOIN_CTAS_PER_SM);
     const int grid = std::min(sm_count() * per_sm, a.max_ctas);
-    kern<<<grid, jn_threads<K>() + 32, smem, st>>>(a);
+    kern<<<grid, jn_threads<K>(NG) + JOIN_PLANNERS<NG>, smem, st>>>(a);
     PJ_CUDA(cudaGetLastError());
     // fix-up: dense output and the true count
     const int fix_threads = std::min(MAX_FIXUP_CTAS, (grid + 31) / 32 * 32);
@@ -1986,14 +1987,14 @@ pj_status large_batch_run_t(const LargeBatch& lb, void* ws, uint32_t* status, cu
         const size_t smem = JoinSmem<K, TABLE_BUCKET>::bytes(a.cap, a.nb_log2);
         PJ_CUDA(set_smem(kern, smem));
         int per_sm = 0;
-        PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, jn_threads<K>() + 32, smem));
+        PJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, jn_threads<K>(1), smem));
         per_sm = std::min(std::max(per_sm, 1), MAX_JOIN_CTAS_PER_SM);
-        kern<<<sm_count() * per_sm, jn_threads<K>() + 32, smem, st>>>(a);
+        kern<<<sm_count() * per_sm, jn_threads<K>(1), smem, st>>>(a);
         PJ_CUDA(cudaGetLastError());
         return PJ_OK;
     };
-    if (lb.unique) return launch(join_kernel<K, TABLE_BUCKET, true, true, false, jn_threads<K>(), 1, true>);
-    return launch(join_kernel<K, TABLE_BUCKET, false, false, false, jn_threads<K>(), 1, true>);
+    if (lb.unique) return launch(join_kernel<K, TABLE_BUCKET, true, true, false, jn_threads<K>(1), 1, true>);
+    return launch(join_kernel<K, TABLE_BUCKET, false, false, false, jn_threads<K>(1), 1, true>);
 }
 
 }  // namespace

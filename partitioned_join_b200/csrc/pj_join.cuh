@@ -437,7 +437,7 @@ constexpr int JOIN_BU = 4;       // build tuples in flight per thread
 constexpr uint32_t JOIN_STEP = 128;  // tuples a warp takes at a time (32 lanes x JOIN_U = JOIN_BU)
 static_assert(JOIN_U * 32 == JOIN_STEP && JOIN_BU * 32 == JOIN_STEP, "a step is U tuples a lane");
 
-// One work item.  A warp of its own works out the next one while the current one probes,
+// One work item.  The next one is worked out while the current one probes,
 // so an item starts without a chain of dependent global loads (item ->
 // partition -> offsets).
 struct ItemMeta {
@@ -507,8 +507,13 @@ struct JoinSmem {
     __host__ __device__ static size_t bytes(int cap, int nb_log2) { return table_bytes(cap, nb_log2); }
 };
 
+// Threads of a join CTA beside the working ones: a planner warp where a
+// partition has several ranges.
+template <int NG>
+constexpr int JOIN_PLANNERS = NG > 1 ? 32 : 0;
+
 template <typename K, int TABLE, bool UNIQUE, bool HASH_SPLIT, bool SLOT_REF, int THREADS, int NG, bool BATCH = false>
-__global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
+__global__ void __launch_bounds__(THREADS + JOIN_PLANNERS<NG>, 1) join_kernel(JoinArgs a)
 {
     using TV = TupleView<K>;
     using Cmp = typename TV::Cmp;
@@ -517,10 +522,15 @@ __global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
     constexpr int NWARPS = THREADS / 32;
     const int lane = threadIdx.x & 31;
     constexpr int U = JOIN_U;
-    // The block's last warp works out the next item while the others build and
-    // probe: inside their loop its code cost them the registers they spilled.
-    const bool planner = threadIdx.x >= THREADS;
-    constexpr int BAR_WORK = 1, BAR_BUILT = 2;  // named barriers: the working warps; they and the planner
+    // Several ranges: the block's last warp works out the next item while the
+    // others build and probe; inside their loop its code cost them the registers
+    // they spilled.  One range: thread 0 does it between build and probe, and
+    // all 24 warps work (with one of them a planner, 2^24 x 2^26 int64 605 us, not
+    // 579; 2^24 x 2^24 int32, four rows a key, 488 and 474).
+    constexpr bool PLANNER = JOIN_PLANNERS<NG> > 0;
+    const bool planner = PLANNER ? threadIdx.x >= THREADS : threadIdx.x == 0;
+    // named barriers: the working warps (all of them without a planner); they and the planner
+    constexpr int BAR_WORK = PLANNER ? 1 : 0, BAR_BUILT = 2;
 
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* table = smem;
@@ -548,7 +558,7 @@ __global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
     const int64_t total_items = a.item_off[a.P];
     const bool write_out = a.out_build != nullptr;
 
-    // The planner warp: item `it` as the next item.  prev_p: the build tuples are fetched
+    // The planner: item `it` as the next item.  prev_p: the build tuples are fetched
     // into L2 unless that partition's are there already (COMPACT tables: see
     // the call).
     auto load_meta = [&](int64_t it, int prev_p) {
@@ -626,7 +636,7 @@ __global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
             s_q = 0;
             s_next = it = static_cast<int64_t>(atomicAdd(a.queue, 1u));
         }
-        it = __shfl_sync(0xffffffffu, it, 0);
+        if constexpr (PLANNER) it = __shfl_sync(0xffffffffu, it, 0);
         if (it < total_items && it < a.max_items) load_meta(it, -1);
     }
     if (threadIdx.x < OUT_SLOTS) s_cslot[threadIdx.x] = ~0ull;
@@ -787,16 +797,12 @@ __global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
             }
             int64_t next = 0;
             if (lane == 0) s_next = next = static_cast<int64_t>(atomicAdd(a.queue, 1u));  // claim the next item early
-            next = __shfl_sync(0xffffffffu, next, 0);
-            // The next item's build side streams into L2 while this item probes,
-            // so the next build's count pass reads L2 (BUCKET tables: 8% at
-            // 2^25; EXACT tables: 2^27 x 2^27 int32 join 1.72 -> 1.59 ms).  Not
-            // for COMPACT tables: their fingerprint checks re-read build tuples
-            // and the prefetched ranges were evicted before use (0.83 GB more
-            // DRAM reads at 2^27 x 2^27, no time gained).
-            asm volatile("bar.sync %0, %1;" ::"n"(BAR_BUILT), "n"(THREADS + 32) : "memory");
-            if (next < total_items && next < a.max_items) load_meta(next, s_meta.p);
-            continue;
+            if constexpr (PLANNER) {
+                next = __shfl_sync(0xffffffffu, next, 0);
+                asm volatile("bar.sync %0, %1;" ::"n"(BAR_BUILT), "n"(THREADS + 32) : "memory");
+                if (next < total_items && next < a.max_items) load_meta(next, s_meta.p);
+                continue;
+            }
         }
         const uint32_t piece = static_cast<uint32_t>(s_meta.piece);
         const int sbits = s_meta.sbits;
@@ -950,29 +956,48 @@ __global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
             part_sync<THREADS, BAR_WORK>();
         }
 
-        // (the planner may fetch the next item's build side now)
-        asm volatile("bar.arrive %0, %1;" ::"n"(BAR_BUILT), "n"(THREADS + 32) : "memory");
+        // The next item's build side streams into L2 while this item probes,
+        // so the next build's count pass reads L2 (BUCKET tables: 8% at
+        // 2^25; EXACT tables: 2^27 x 2^27 int32 join 1.72 -> 1.59 ms).  Not
+        // for COMPACT tables: their fingerprint checks re-read build tuples
+        // and the prefetched ranges were evicted before use (0.83 GB more
+        // DRAM reads at 2^27 x 2^27, no time gained).
+        if constexpr (PLANNER)
+            asm volatile("bar.arrive %0, %1;" ::"n"(BAR_BUILT), "n"(THREADS + 32) : "memory");
+        else if (planner && s_next < total_items && s_next < a.max_items)
+            load_meta(s_next, s_meta.p);
 
         // ---- probe: warps run independently; loads run one step ahead ----
         if (!skip_item) {
             // warps claim steps of 32*U tuples from a shared counter, so they
             // finish the item together; the next claim's loads run ahead
-            const uint32_t qn = s_qst.last[NG - 1];
+            // One range: its start and length stay in registers and a step is its
+            // first tuple (read from shared memory at every step, the loads
+            // waited for them: 2^24 x 2^24 int64, four rows a key, 578 -> 517 us).
+            const uint32_t qn = NG == 1 ? s_qst.n[0] : s_qst.last[NG - 1];
+            const uint32_t* qbase = a.probe_tuples + static_cast<size_t>(s_qst.start[0]) * TV::WORDS;
             uint32_t nh[U];
             Cmp nk[U];
             int32_t nr[U];
             auto claim = [&]() -> uint32_t {
                 uint32_t st = 0;
                 if (lane == 0) st = atomicAdd(&s_step, 1u);
-                return __shfl_sync(0xffffffffu, st, 0);
+                return __shfl_sync(0xffffffffu, st, 0) * (NG == 1 ? JOIN_STEP : 1u);
             };
             StepCursor<NG, TV::WORDS> cur;
             auto load_step = [&](uint32_t st) {
-                int left;
-                const uint32_t* t = cur.at(s_qst, a.probe_tuples, st, left);
+                if constexpr (NG == 1) {
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    TV::load_stream_if(t, u * 32, u * 32 < left, nh[u], nk[u], nr[u], stream_pol);
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t i = st + u * 32 + lane;
+                        TV::load_stream_if(qbase, i, i < qn, nh[u], nk[u], nr[u], stream_pol);
+                    }
+                } else {
+                    int left;
+                    const uint32_t* t = cur.at(s_qst, a.probe_tuples, st, left);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        TV::load_stream_if(t, u * 32, u * 32 < left, nh[u], nk[u], nr[u], stream_pol);
                 }
             };
             uint32_t s0 = claim();
@@ -1270,7 +1295,6 @@ __global__ void __launch_bounds__(THREADS + 32, 1) join_kernel(JoinArgs a)
                             emit[u] = lookup(u, at_u, end_u, sl_u, steps_u, live_u, brow[u]);
                         }
                     }
-                    __syncwarp();
                     append_direct(emit, brow, r);
                 } else {
                     // repeated build keys: every tuple walks on, one match per lane per append
