@@ -321,9 +321,11 @@ pj_status pj_partition(const void* keys, int64_t n, int32_t key_bytes, const pj_
  * Joins with unique build keys of up to 2^22 rows are joined through hash
  * tables in L2, a group of joins at a time: one launch builds the group's
  * tables, one probes them, every match written at an exact position of its
- * join's output (large_batched = 1).  Of the others, joins whose build side
- * fits one shared-memory table skip partitioning: one persistent kernel drains a (join, probe chunk) work queue over all of
- * them, writing each join's pairs densely to its own output.  Larger joins
+ * join's output (large_batched = 1) -- except those with so few probe rows
+ * that a table does not pay, if enough of them come together.  Of the others,
+ * joins whose build side fits one shared-memory table skip partitioning: one
+ * persistent kernel drains a (join, probe chunk) work queue over all of them,
+ * writing each join's pairs densely to its own output.  Larger joins
  * (up to 2^10 partitions each) are partitioned together -- one histogram,
  * one scan and one scatter launch over both key columns of all of them --
  * and joined by one persistent launch that drains a (join, partition, probe

@@ -275,10 +275,10 @@ def generate_tables(n_build: int, n_probe: int, key_dtype=torch.int32, rand_max:
 
 class BatchJoiner:
     """A batch of joins (pj_join_batch): joins of up to 2^22 unique build rows
-    run through hash tables in L2, a group of joins per launch; of the others,
-    those whose build side fits one shared-memory table run in one persistent
-    launch draining a (join, probe chunk) queue, the rest take the partitioned
-    path.  Outputs and the
+    run through hash tables in L2, a group of joins per launch (unless too few
+    probe rows come with them); of the others, those whose build side fits one
+    shared-memory table run in one persistent launch draining a (join, probe
+    chunk) queue, the rest take the partitioned path.  Outputs and the
     workspace are allocated once; launch() only enqueues kernels, so it can
     be captured in a CUDA graph (see graph())."""
 

@@ -4,7 +4,8 @@
 // (pj_join_batch) is split by kind and size:
 //   * joins with unique build keys of up to 2^22 rows (large_batched = 1, the
 //     default) take the tables of pj_global.cuh: groups of joins whose tables
-//     together stay in L2, one build and one probe launch a group.
+//     together stay in L2, one build and one probe launch a group -- unless
+//     they have too few probe rows for a table's build (table_joins).
 // The others:
 //   * direct joins -- build side no larger than one shared-memory table --
 //     skip partitioning altogether.  One persistent kernel drains a queue of
@@ -241,14 +242,72 @@ __global__ void __launch_bounds__(THREADS) batch_direct_kernel(const BatchJob* _
 // Host side.
 
 struct Split {
-    std::vector<int> direct, large;
+    std::vector<int> global, direct, large;
 };
 
-// Joins that take a table of pj_global.cuh.
-bool takes_global(const pj_join_desc& d, const pj_batch_config& cfg)
+// Joins that can take a table of pj_global.cuh.
+bool may_take_table(const pj_join_desc& d, const pj_batch_config& cfg)
 {
     return cfg.large_batched && d.unique_build_keys && d.n_build > 0 && d.n_build <= GT_MAX_BUILD && d.n_probe > 0 &&
            d.n_probe <= INT32_MAX;
+}
+
+// What a join saves off the tables, in picoseconds.  A table's inserts are its
+// cost: 2^24 4-byte build rows in all and few probe rows take 430 us by tables,
+// 160 direct (builds of 2^13) and 230 partitioned together (2^20); 8-byte rows,
+// whose slots are half the size, 330, 165 and 346.  A probe row costs 4 ps
+// less by a table (2^24 build, 2^28 probe rows: 2.57 ms, 3.48 partitioned).
+int64_t gain_off_table(const pj_join_desc& d, bool direct)
+{
+    // (8-byte joins of a few partitions are slow to partition: 2^9 of 2^15 rows
+    // 463 us, 2^7 of 2^17 rows 354)
+    const int64_t build = d.key_bytes == 4 ? (direct ? 16 : 15) : direct ? 10 : d.n_build >= (1 << 17) ? 3 : 0;
+    return build * d.n_build - 4 * d.n_probe;
+}
+// Savings that pay for launches beside those of the tables: partitioning takes a
+// dozen (64 joins of 2^17 x 2^17 4-byte rows, 92 us by the above: 306 us by
+// tables, 250 partitioned; 8 of 2^19 x 2^18, 55: 141 and 123; 8 of 2^17 x 2^17,
+// 12: 59 and 105), the direct kernel two.
+constexpr int64_t PARTITION_GAIN = 60 * int64_t(1000000);
+constexpr int64_t DIRECT_GAIN = 8 * int64_t(1000000);
+
+// The joins that take a table: those with too few probe rows for its build go
+// the other routes, if together they save more than the launches cost.
+std::vector<char> table_joins(const pj_join_desc* descs, int32_t n, const pj_batch_config& cfg)
+{
+    std::vector<char> table(std::max(n, 0), 0);
+    bool repeated = false, any_direct = false, any_large = false;
+    bool stays = false;  // a join that takes a table in any case
+    bool few = true;     // no join to go direct has more probe than build rows
+    int64_t direct_gain = 0, large_gain = 0;
+    auto direct = [&](const pj_join_desc& d) { return d.n_build <= cfg.direct_max_build; };
+    for (int i = 0; i < n; ++i) {
+        const pj_join_desc& d = descs[i];
+        if (d.n_build <= 0 || d.n_probe <= 0) continue;
+        repeated = repeated || !d.unique_build_keys;
+        if (!may_take_table(d, cfg)) {
+            (direct(d) ? any_direct : any_large) = true;
+            continue;
+        }
+        table[i] = 1;
+        const int64_t g = gain_off_table(d, direct(d));
+        if (g <= 0) {
+            stays = true;
+        } else if (direct(d)) {
+            direct_gain += g;
+            few = few && d.n_probe <= d.n_build;
+        } else {
+            large_gain += g;
+        }
+    }
+    // (repeated keys among them would cost the others the kernel for unique ones)
+    const bool large_moves = large_gain > 0 && !repeated && (any_large || large_gain >= PARTITION_GAIN);
+    stays = stays || (large_gain > 0 && !large_moves);
+    const bool direct_moves = direct_gain >= DIRECT_GAIN || (direct_gain > 0 && (any_direct || (!stays && few)));
+    for (int i = 0; i < n; ++i)
+        if (table[i] && gain_off_table(descs[i], direct(descs[i])) > 0 && (direct(descs[i]) ? direct_moves : large_moves))
+            table[i] = 0;
+    return table;
 }
 
 // Buckets of such a table: two rows a bucket of four slots, three of eight.
@@ -270,10 +329,11 @@ constexpr int64_t GLOBAL_SMALL_PROBE = int64_t(1) << 21;
 Split split_batch(const pj_join_desc* descs, int32_t n, const pj_batch_config& cfg)
 {
     Split s;
+    const std::vector<char> table = table_joins(descs, n, cfg);
     for (int i = 0; i < n; ++i) {
         const pj_join_desc& d = descs[i];
-        if (takes_global(d, cfg)) continue;
-        if (d.n_build <= cfg.direct_max_build && d.n_build > 0 && d.n_probe > 0) s.direct.push_back(i);
+        if (table[i]) s.global.push_back(i);
+        else if (d.n_build <= cfg.direct_max_build && d.n_build > 0 && d.n_probe > 0) s.direct.push_back(i);
         else s.large.push_back(i);
     }
     return s;
@@ -301,7 +361,7 @@ struct GlobalGroup {
 
 struct BatchLayout {
     size_t ctrl = 0, jobs = 0, large = 0, large_bytes = 0, batched = 0, total = 0;
-    std::vector<int> global;             // joins by global tables
+    Split split;                         // the joins by route
     std::vector<GlobalGroup> groups;
     size_t gjobs = 0, gitems = 0, region = 0;
     uint32_t n_gitems = 0;
@@ -318,7 +378,8 @@ pj_status layout_for(const pj_join_desc* descs, int32_t n, const pj_batch_config
     b.ctrl = 0;
     b.jobs = 256;
     b.large = align256(b.jobs + sizeof(BatchJob) * static_cast<size_t>(std::max(n, 1)));
-    const Split sp = split_batch(descs, n, cfg);
+    b.split = split_batch(descs, n, cfg);
+    const Split& sp = b.split;
     if (cfg.large_batched) {
         pj_status s = pj_internal::large_batch_layout(descs, sp.large, cfg.large_bits_delta, &b.lb);
         if (s != PJ_OK) return s;
@@ -337,42 +398,57 @@ pj_status layout_for(const pj_join_desc* descs, int32_t n, const pj_batch_config
     }
     b.batched = b.large + align256(b.large_bytes);
     b.gjobs = b.batched + align256(b.lb.total);
-    uint32_t bi = 0, pi = 0;
-    size_t most = 0;
-    int64_t build_rows = 0, probe_rows = 0;
-    for (int i = 0; i < n; ++i)
-        if (takes_global(descs[i], cfg)) {
+    // Groups of the joins that take tables.  The room is that of all joins that
+    // could, so that it does not depend on where the direct path ends.
+    auto group = [&](const std::vector<int>& joins, std::vector<GlobalGroup>& groups, uint32_t& n_items) {
+        int64_t build_rows = 0, probe_rows = 0;
+        for (int i : joins) {
             build_rows += descs[i].n_build;
             probe_rows += descs[i].n_probe;
         }
-    if (build_rows < GLOBAL_SMALL_BUILD) b.build_item = GT_THREADS;
-    if (probe_rows < GLOBAL_SMALL_PROBE) b.probe_item = GT_TILE;
-    for (int i = 0; i < n; ++i) {
-        const pj_join_desc& d = descs[i];
-        if (!takes_global(d, cfg)) continue;
-        if (!d.build_keys || !d.probe_keys) return PJ_ERR_INVALID;
-        const size_t bytes = 32 * static_cast<size_t>(global_buckets(d));
-        if (b.groups.empty() || b.groups.back().bytes + bytes > GLOBAL_GROUP_BYTES) {
-            GlobalGroup g;
-            g.b0 = bi;
-            g.p0 = pi;
-            b.groups.push_back(g);
+        b.build_item = build_rows < GLOBAL_SMALL_BUILD ? GT_THREADS : GT_BUILD_ITEM;
+        b.probe_item = probe_rows < GLOBAL_SMALL_PROBE ? GT_TILE : GT_PROBE_ITEM;
+        uint32_t bi = 0, pi = 0;
+        size_t most = 0;
+        for (int i : joins) {
+            const pj_join_desc& d = descs[i];
+            const size_t bytes = 32 * static_cast<size_t>(global_buckets(d));
+            if (groups.empty() || groups.back().bytes + bytes > GLOBAL_GROUP_BYTES) {
+                GlobalGroup g;
+                g.b0 = bi;
+                g.p0 = pi;
+                groups.push_back(g);
+            }
+            GlobalGroup& g = groups.back();
+            const uint32_t nbi = static_cast<uint32_t>((d.n_build + b.build_item - 1) / b.build_item);
+            const uint32_t npi = static_cast<uint32_t>((d.n_probe + b.probe_item - 1) / b.probe_item);
+            bi += nbi;
+            pi += npi;
+            g.nb += nbi;
+            g.np += npi;
+            g.bytes += bytes;
+            most = std::max(most, g.bytes);
         }
-        GlobalGroup& g = b.groups.back();
-        const uint32_t nbi = static_cast<uint32_t>((d.n_build + b.build_item - 1) / b.build_item);
-        const uint32_t npi = static_cast<uint32_t>((d.n_probe + b.probe_item - 1) / b.probe_item);
-        bi += nbi;
-        pi += npi;
-        g.nb += nbi;
-        g.np += npi;
-        g.bytes += bytes;
-        most = std::max(most, g.bytes);
-        b.global.push_back(i);
+        for (GlobalGroup& g : groups) g.p0 += bi;  // the probe items follow all build items
+        n_items = bi + pi;
+        return most;
+    };
+    std::vector<int> could;
+    for (int i = 0; i < n; ++i)
+        if (may_take_table(descs[i], cfg)) {
+            if (!descs[i].build_keys || !descs[i].probe_keys) return PJ_ERR_INVALID;
+            could.push_back(i);
+        }
+    const size_t most = group(could, b.groups, b.n_gitems);
+    size_t room = b.n_gitems;
+    if (!could.empty())  // (fewer rows may mean small items, but then there are few)
+        room = std::max<size_t>(room, GLOBAL_SMALL_BUILD / GT_THREADS + GLOBAL_SMALL_PROBE / GT_TILE + 2 * could.size());
+    if (could.size() != sp.global.size()) {
+        b.groups.clear();
+        group(sp.global, b.groups, b.n_gitems);
     }
-    for (GlobalGroup& g : b.groups) g.p0 += bi;  // the probe items follow all build items
-    b.n_gitems = bi + pi;
-    b.gitems = b.gjobs + align256(sizeof(GtJob) * b.global.size());
-    b.region = b.gitems + align256(sizeof(GtItem) * static_cast<size_t>(b.n_gitems));
+    b.gitems = b.gjobs + align256(sizeof(GtJob) * could.size());
+    b.region = b.gitems + align256(sizeof(GtItem) * room);
     b.total = b.region + align256(most);
     *L = std::move(b);
     return PJ_OK;
@@ -462,7 +538,7 @@ pj_status run_batch(const pj_join_desc* descs, const pj_output* outs, int32_t n,
     uint32_t* status = reinterpret_cast<uint32_t*>(w + L.ctrl);
     uint32_t* queue = status + 1;
     if (cudaMemsetAsync(queue, 0, sizeof(uint32_t), st) != cudaSuccess) return PJ_ERR_CUDA;
-    const Split sp = split_batch(descs, n, cfg);
+    const Split& sp = L.split;
     const BatchJob* jobs = reinterpret_cast<const BatchJob*>(w + L.jobs);
     if ((parts & 1) && !sp.direct.empty()) {
         const int nd = static_cast<int>(sp.direct.size());
@@ -472,7 +548,7 @@ pj_status run_batch(const pj_join_desc* descs, const pj_output* outs, int32_t n,
                                     : launch_direct_k<int64_t>(jobs, nd, items, cfg, queue, status, st);
         if (s != PJ_OK) return s;
     }
-    if ((parts & 2) && !L.global.empty()) {
+    if ((parts & 2) && !L.split.global.empty()) {
         s = descs[0].key_bytes == 4 ? launch_global<int32_t>(L, w, status, st) : launch_global<int64_t>(L, w, status, st);
         if (s != PJ_OK) return s;
     }
@@ -531,7 +607,7 @@ pj_status pj_batch_prepare(const pj_join_desc* descs, const pj_output* outs, int
     BatchLayout L;
     if ((s = layout_for(descs, n, *cfg, &L)) != PJ_OK) return s;
     if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u) || ws_bytes < L.total) return PJ_ERR_WORKSPACE;
-    const Split sp = split_batch(descs, n, *cfg);
+    const Split& sp = L.split;
     std::vector<BatchJob> jobs;
     int64_t item = 0;
     for (int i : sp.direct) {
@@ -560,11 +636,11 @@ pj_status pj_batch_prepare(const pj_join_desc* descs, const pj_output* outs, int
         return PJ_ERR_CUDA;
     std::vector<GtJob> gjobs;
     std::vector<GtItem> gitems(L.n_gitems);
-    if (!L.global.empty()) {
+    if (!L.split.global.empty()) {
         uint32_t bi = 0, pi = L.groups[0].p0;
         size_t group = 0, left = L.groups[0].nb;  // build items left in the current group
         uint32_t bucket = 0;
-        for (int i : L.global) {
+        for (int i : L.split.global) {
             const pj_join_desc& d = descs[i];
             if (left == 0) {
                 left = L.groups[++group].nb;
