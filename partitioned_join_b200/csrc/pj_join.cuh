@@ -926,16 +926,14 @@ __global__ void __launch_bounds__(THREADS + JOIN_PLANNERS<NG>, 1) join_kernel(Jo
                 else orows[i] = EMPTY_ROW;
             }
             part_sync<THREADS, BAR_WORK>();
-            StepCursor<NG, TV::WORDS> cur;
-            for (uint32_t s4 = warp; s4 < b_total * JOIN_BU; s4 += NWARPS) {
-                uint32_t h = 0;
+            // (OPEN tables: one range)
+            const uint32_t* bbase = a.build_tuples + static_cast<size_t>(s_bst.start[0]) * TV::WORDS;
+            const uint32_t bn = s_bst.n[0];
+            for (uint32_t i = threadIdx.x; i < bn; i += THREADS) {
+                uint32_t h;
                 Cmp k;
-                int32_t r = -1;
-                __syncwarp();
-                int left;
-                const uint32_t* t = cur.at(s_bst, a.build_tuples, s4 / JOIN_BU, left);
-                const int i = (s4 % JOIN_BU) * 32;
-                if (i < left) TV::load(t, i, h, k, r);
+                int32_t r;
+                TV::load(bbase, i, h, k, r);
                 if (r < 0 || !in_piece(h)) continue;
                 uint32_t sl = slot_of(h);
                 int tries = 0;
