@@ -718,17 +718,38 @@ pj_status launch_scatter_units(const K* keys, int64_t n, int64_t chunk, int item
     return PJ_OK;
 }
 
+template <typename K, int W, bool HASHD, bool HEAVY>
+pj_status launch_scatter_rounds(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P,
+                                const int64_t* offsets, uint32_t* out, uint32_t cap32, uint32_t* status,
+                                const HeavyCtx& hc, cudaStream_t st)
+{
+    constexpr int V = sc_v<K>();
+    auto* kern = scatter_rounds_kernel<K, SC_THREADS, V, W, HASHD, HEAVY>;
+    constexpr int TW = WcTraits<K, W>::TW;
+    const int cap = wc_cap(sizeof(K), W, P, SC_THREADS * V, HEAVY ? HeavyTable::BYTES + 16 : 0);
+    const size_t smem = HEAVY ? heavy_table_offset(P, cap * TW) + HeavyTable::BYTES : scatter_smem(sizeof(K), cap, P);
+    PJ_CUDA(set_smem(kern, smem));
+    typename HeavyArg<HEAVY>::type h{};
+    if constexpr (HEAVY) h = *hc.hs;
+    kern<<<items, SC_THREADS, smem, st>>>(keys, n, chunk, items, f, P, cap, offsets, out, cap32, status, h, hc.out);
+    PJ_CUDA(cudaGetLastError());
+    return PJ_OK;
+}
+
 template <typename K, bool HASHD, bool HEAVY>
 pj_status launch_scatter_t(const K* keys, int64_t n, int64_t chunk, int items, DigitFn f, int P, int W, int ipg,
                            const int64_t* offsets, uint32_t* out, int64_t out_cap, uint32_t* status,
                            const HeavyCtx& hc, cudaStream_t st)
 {
-    typename HeavyArg<HEAVY>::type h{};
-    if constexpr (HEAVY) h = *hc.hs;
     const uint32_t cap32 = static_cast<uint32_t>(std::min<int64_t>(out_cap, UINT32_MAX));
     constexpr int V = sc_v<K>();
+    constexpr int U_SECTOR = WcUnits<K>::CH;  // tuples of a sector
     const int lf = unit_logf<K>(P, W, SC_THREADS, V, HEAVY ? HeavyTable::BYTES + 16 : 0, chunk);
-    if (lf >= 0) {
+    // 4096 partitions of a few tuples of an item each: clearing and closing a
+    // unit for each costs more than the barriers of the form with rounds (2^10
+    // int32 keys 59 -> 43 us, 2^22 93 -> 80; 2^24, 28 tuples each, 165 by units, 172)
+    const bool few = P >= 4096 && W == U_SECTOR && ipg == items && chunk < 16 * static_cast<int64_t>(P);
+    if (lf >= 0 && !few) {
         // 8-byte keys over 4096 partitions: two tuples a unit, and HBM takes the
         // sectors no faster than half the warps bring them (2^28 keys 2.40 ->
         // 2.16 ms); fewer partitions wait on the warps (2048: 434 -> 473 us), as
@@ -740,17 +761,10 @@ pj_status launch_scatter_t(const K* keys, int64_t n, int64_t chunk, int items, D
         return launch_scatter_units<K, SC_THREADS, HASHD, HEAVY>(keys, n, chunk, items, f, P, lf, W, ipg, offsets, out,
                                                                  cap32, status, hc, st);
     }
-    if constexpr (sizeof(K) == 4) {  // 8192 partitions of half-sector groups
-        if (W != 2 || ipg != items) return PJ_ERR_INVALID;
-        auto* kern = scatter_rounds_kernel<K, SC_THREADS, V, 2, HASHD, HEAVY>;
-        constexpr int TW = WcTraits<K, 2>::TW;
-        const int cap = wc_cap(sizeof(K), W, P, SC_THREADS * V, HEAVY ? HeavyTable::BYTES + 16 : 0);
-        const size_t smem = HEAVY ? heavy_table_offset(P, cap * TW) + HeavyTable::BYTES : scatter_smem(sizeof(K), cap, P);
-        PJ_CUDA(set_smem(kern, smem));
-        kern<<<items, SC_THREADS, smem, st>>>(keys, n, chunk, items, f, P, cap, offsets, out, cap32, status, h, hc.out);
-        PJ_CUDA(cudaGetLastError());
-        return PJ_OK;
-    }
+    if (ipg != items) return PJ_ERR_INVALID;
+    if (W == U_SECTOR) return launch_scatter_rounds<K, U_SECTOR, HASHD, HEAVY>(keys, n, chunk, items, f, P, offsets, out, cap32, status, hc, st);
+    if constexpr (sizeof(K) == 4)  // 8192 partitions of half-sector groups
+        if (W == 2) return launch_scatter_rounds<K, 2, HASHD, HEAVY>(keys, n, chunk, items, f, P, offsets, out, cap32, status, hc, st);
     return PJ_ERR_INVALID;
 }
 

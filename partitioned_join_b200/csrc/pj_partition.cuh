@@ -974,8 +974,8 @@ __device__ __forceinline__ void heavy_take(const HeavyTable& heavy, const K (&ke
 }
 
 // Scatter of a raw key column (row = key index).  V keys per thread per
-// round (whole 16-byte vectors), the next two rounds' vectors loaded while
-// the current round is placed; the warps of the CTA run on their own.
+// round (whole 16-byte vectors), the next round's vectors loaded while the
+// current one is placed; the warps of the CTA run on their own.
 template <typename K, int THREADS, int V, bool HASHD, bool HEAVY>
 __global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __restrict__ keys, int64_t n,
                                                                   int64_t chunk, int32_t n_items, DigitFn f,
@@ -1091,11 +1091,12 @@ __global__ void __launch_bounds__(THREADS, 1) scatter_keys_kernel(const K* __res
     }
 }
 
-// The same scatter with wc_place, for fan-outs whose units and cursors do not
-// fit shared memory (8192 partitions of half-sector groups).  V keys per thread per
-// round (whole 16-byte vectors), the next two rounds' vectors loaded while
-// the current round is processed.  Per partition the CTA keeps a buffer of
-// cap tuples (whole groups of W), a fill count and an output cursor.
+// The same scatter with wc_place, in rounds between block barriers: for
+// fan-outs whose units and cursors do not fit shared memory (8192 partitions of
+// half-sector groups), and for 4096 partitions of items with few tuples.  V
+// keys per thread per round (whole 16-byte vectors), the next round's vectors
+// loaded while the current one is processed.  Per partition the CTA keeps a
+// buffer of cap tuples (whole groups of W), a fill count and an output cursor.
 template <typename K, int THREADS, int V, int W, bool HASHD, bool HEAVY>
 __global__ void __launch_bounds__(THREADS, 1) scatter_rounds_kernel(const K* __restrict__ keys, int64_t n,
                                                                   int64_t chunk, int32_t n_items, DigitFn f,
