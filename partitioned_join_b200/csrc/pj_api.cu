@@ -43,7 +43,12 @@ constexpr int HEAVY_MIN_SAMPLES = 32;      // a heavy key holds >= 1/2048 of the
 constexpr int64_t HEAVY_MIN_PROBE = 1 << 20;  // smaller probe sides: no heavy-key path
 constexpr double HEAVY_MIN_SHARE = 0.5;       // share of the probe rows the heavy keys must hold
 constexpr int64_t GLOBAL_MAX_BUILD = GT_MAX_BUILD;  // build rows of a join by one table in L2
-constexpr int64_t GLOBAL_SPARSE_BUILD = 1 << 20;  // up to here its table has four slots a row
+// Up to here the table has one row a bucket, beyond two or three: lookups end in
+// the first bucket and a tag rarely fits another key, until the table and the
+// build keys outgrow L2.  Builds with four probe rows a row, one a bucket and
+// more: 4-byte keys 2^20 rows 68 and 84 us, 2^21 113 and 131, 2^21.5 193 and 168;
+// 8-byte keys 2^20 72 and 80, 2^20.5 94 and 98, 2^21 131 and 125.
+constexpr int64_t GLOBAL_SPARSE_32 = 1 << 21, GLOBAL_SPARSE_64 = 3 << 19;
 constexpr int64_t GROUP_BYTES = int64_t(256) << 20;  // tuples of one item group (pj_partition.cuh)
 constexpr size_t LEARN_BYTES = 4096;          // features, activations and scores of the learned planner
 
@@ -1036,11 +1041,12 @@ GlobalPlan global_plan(const pj_join_desc* d, const pj_plan* p, const Layout& L)
     g.table = o;
     if (d->unique_build_keys) {
         // four 8-byte slots (4-byte keys) or eight 4-byte slots (8-byte keys)
-        // a bucket.  One row a bucket while the table stays small; beyond, two
+        // a bucket.  One row a bucket while all stays in L2; beyond, two
         // rows (three for 8-byte keys: 14 % of four-slot buckets are full at
         // two, 1 % of eight-slot ones at three) to keep it and the build keys
         // in L2.
-        const int64_t per = n <= GLOBAL_SPARSE_BUILD ? 1 : d->key_bytes == 4 ? 2 : 3;
+        const int64_t sparse = d->key_bytes == 4 ? GLOBAL_SPARSE_32 : GLOBAL_SPARSE_64;
+        const int64_t per = n <= sparse ? 1 : d->key_bytes == 4 ? 2 : 3;
         const int64_t slots = d->key_bytes == 4 ? 4 : 8;
         const int64_t want = std::max<int64_t>(8, (n + per - 1) / per);
         const int64_t fit = static_cast<int64_t>((L.total - o) / 32);
