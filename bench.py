@@ -732,6 +732,15 @@ def run_batch(args, rank, world, local, emit=True):
     bj.check()
     graph_ok = verify_all(bj.build_row, bj.probe_row, bj.count)
     best_ms = min(batch_ms, tuned_ms, graph_ms)
+    # (four probe rows a build row: joins of up to 2^22 unique build rows take tables in L2)
+    paths = {"tables_in_l2": 0, "direct": 0, "partitioned_together": 0, "one_after_another": 0}
+    for b, _ in pairs:
+        if bj.config.large_batched and b.numel() <= 1 << 22:
+            paths["tables_in_l2"] += 1
+        elif b.numel() <= bj.config.direct_max_build:
+            paths["direct"] += 1
+        else:
+            paths["partitioned_together" if bj.config.large_batched else "one_after_another"] += 1
     line = {
         "metric": "tuples/s, 512-join uneven batch (cfg5)", "value": tuples / (best_ms / 1e3), "unit": UNIT,
         "n_gpus": world, "steps": steps, "warmup": args.warmup, "ms_per_step": best_ms, "higher_is_better": True,
@@ -744,9 +753,7 @@ def run_batch(args, rank, world, local, emit=True):
                         "batch_autotuned_graph": graph_ms, "autotuner_estimate": tuned_ms_est},
         "speedup_vs_plain": plain_ms / best_ms,
         "speedup_vs_plain_autotuned": plain_tuned_ms / best_ms,
-        "joins_by_path": {"direct": int(sum(1 for b, _ in pairs if 0 < b.numel() <= bj.config.direct_max_build)),
-                          "partitioned_together": int(sum(1 for b, _ in pairs if b.numel() > bj.config.direct_max_build))
-                          if bj.config.large_batched else 0},
+        "joins_by_path": paths,
         "verified": {"plain": plain_ok, "plain_autotuned": plain_tuned_ok, "batch": batch_ok, "graph": graph_ok},
     }
     if rank == 0 and emit:

@@ -222,7 +222,10 @@ enum {
 };
 
 /* pj_inner_join with a cudaEvent around every stage; SYNCHRONISES the
- * stream and writes the milliseconds of each stage to stage_ms[PJ_NUM_STAGES]. */
+ * stream and writes the milliseconds of each stage to stage_ms[PJ_NUM_STAGES].
+ * A join by one table in L2 has two stages: the table's build (clearing
+ * included) counts as PJ_STAGE_BUILD_SCATTER, the lookups and the output as
+ * PJ_STAGE_JOIN, and the others are about 0. */
 pj_status pj_inner_join_timed(const pj_join_desc* desc, const pj_plan* plan, pj_output* out,
                               void* workspace, size_t workspace_bytes, pj_stream stream,
                               float* stage_ms);
