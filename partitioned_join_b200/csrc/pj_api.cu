@@ -1111,7 +1111,10 @@ pj_status run_global(const pj_join_desc* d, const GlobalPlan& g, const Layout& L
         for (int i = PJ_STAGE_BUILD_PASS2; i <= PJ_STAGE_JOIN; ++i) E.mark(i, st);
         // (the list takes the counts' place: the ranges hold them by now)
         const GtLong later = long_ranges(d->n_build, d->n_probe, d->key_bytes, cursor + 1, counts);
-        PJ_CUDA(launch_after(gt_probe_multi_kernel<K>, pgrid, st, pk, np, bk, range, g.nb, entries, later, o));
+        // (not launched ahead: beside the kernel before it, its CTAs would crowd on the few SMs that one leaves free --
+        // 2^16 x 2^14 4-byte rows, 16 a key, behind other work: 163 us, 48 with an SM each)
+        gt_probe_multi_kernel<K><<<pgrid, GT_THREADS, 0, st>>>(pk, np, bk, range, g.nb, entries, later, o);
+        PJ_CUDA(cudaGetLastError());
         if (nb > GT_LONG) {
             PJ_CUDA(launch_after(gt_probe_long_kernel<K>, static_cast<unsigned>(sm_count()) * GT_LONG_CTAS, st, pk, np, bk,
                                  range, g.nb, entries, later, o));
