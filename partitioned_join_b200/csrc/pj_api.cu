@@ -962,6 +962,7 @@ struct GlobalPlan {
     size_t zeroed = 0;        // workspace bytes to clear, from 0
     size_t table = 0;         // unique: buckets; repeated keys: bucket counts
     size_t range = 0, entries = 0;  // repeated keys
+    bool wide = false;        // repeated 8-byte keys: the entries hold the key
 };
 
 // PJ_PLAN_FLAG_AUTO and, above it, a checksum (FNV-1a) of the fields that say
@@ -1015,13 +1016,13 @@ int64_t long_words(int64_t n_probe) { return (n_probe + 32 * GT_U - 1) / (32 * G
 
 // GtLong of a join: as many bits for the rounds as the words leave, and slices
 // so large that the rounds of any keys fit them (one step up to 2^29 x 2^22 rows).
-GtLong long_ranges(int64_t n_build, int64_t n_probe, int key_bytes, void* cursor, void* list)
+GtLong long_ranges(int64_t n_build, int64_t n_probe, int key_bytes, bool wide, void* cursor, void* list)
 {
     GtLong g;
     g.cursor = static_cast<unsigned long long*>(cursor);
     g.list = static_cast<unsigned long long*>(list);
     const int64_t words = long_words(n_probe);
-    g.walk = n_probe < GT_WALK_PROBE ? GT_LONG : key_bytes == 4 ? GT_WALK_32 : GT_WALK_64;
+    g.walk = n_probe < GT_WALK_PROBE || (key_bytes == 8 && !wide) ? GT_LONG : wide ? GT_WALK_64 : GT_WALK_32;
     g.round_bits = 63 - ilog2_floor(words);
     for (g.slice = GT_SLICE;; g.slice *= 2) {
         const int64_t slices = n_probe * ((n_build + g.slice - 1) / g.slice);  // < 2^46
@@ -1062,8 +1063,49 @@ GlobalPlan global_plan(const pj_join_desc* d, const pj_plan* p, const Layout& L)
     g.zeroed = align_up(o + 4 * static_cast<size_t>(g.nb), 256);
     g.range = std::max(g.zeroed, align_up(o + 8 * static_cast<size_t>(long_words(d->n_probe)), 256));
     g.entries = align_up(g.range + 8 * static_cast<size_t>(g.nb), 256);
-    g.use = g.entries + 8 * static_cast<size_t>(n) <= L.total;
+    auto fits = [&](size_t bytes) { return g.entries + align_up(bytes * static_cast<size_t>(n), 32) <= L.total; };  // whole sectors
+    g.wide = d->key_bytes == 8 && d->n_probe >= n && fits(16);
+    g.use = g.wide || fits(8);
     return g;
+}
+
+// Repeated build keys: the rows grouped by bucket, then the lookups.
+template <typename K, bool WIDE>
+pj_status run_global_repeated(const pj_join_desc* d, const GlobalPlan& g, const Layout& L, uint8_t* ws,
+                              const GlobalOut& o, cudaStream_t st, const StageEvents& E)
+{
+    const K* bk = static_cast<const K*>(d->build_keys);
+    const K* pk = static_cast<const K*>(d->probe_keys);
+    const uint32_t nb = static_cast<uint32_t>(d->n_build), np = static_cast<uint32_t>(d->n_probe);
+    const unsigned bgrid = (nb + GT_THREADS - 1) / GT_THREADS, pgrid = (np + GT_TILE - 1) / GT_TILE;
+    auto* counts = reinterpret_cast<uint32_t*>(ws + g.table);
+    auto* range = reinterpret_cast<uint2*>(ws + g.range);
+    auto* entries = reinterpret_cast<typename GtEntry<K, WIDE>::T*>(ws + g.entries);
+    // (the counter block's words double as 64-bit cursors: entries, and GtLong's)
+    auto* cursor = reinterpret_cast<unsigned long long*>(ws + L.counters);
+    if (d->n_build <= GT_GROUP) {
+        gt_group_kernel<K, WIDE><<<1, GT_GROUP_THREADS, 0, st>>>(bk, nb, g.nb, reinterpret_cast<uint32_t*>(ws),
+                                                           static_cast<int>(L.counters / 4) + 8, range, entries, o.count);
+    } else {
+        gt_count_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, counts, g.nb, o.count);
+        PJ_CUDA(cudaGetLastError());
+        PJ_CUDA(launch_after(gt_alloc_kernel, (g.nb + GT_THREADS * GT_ALLOC - 1) / (GT_THREADS * GT_ALLOC), st, counts,
+                             g.nb, range, cursor));
+        PJ_CUDA(launch_after(gt_place_kernel<K, WIDE>, bgrid, st, bk, nb, range, g.nb, entries));
+    }
+    PJ_CUDA(cudaGetLastError());
+    for (int i = PJ_STAGE_BUILD_PASS2; i <= PJ_STAGE_JOIN; ++i) E.mark(i, st);
+    // (the list takes the counts' place: the ranges hold them by now)
+    const GtLong later = long_ranges(d->n_build, d->n_probe, d->key_bytes, WIDE, cursor + 1, counts);
+    // (not launched ahead: beside the kernel before it, its CTAs would crowd on the few SMs that one leaves free --
+    // 2^16 x 2^14 4-byte rows, 16 a key, behind other work: 79 us, 40 with an SM each)
+    gt_probe_multi_kernel<K, WIDE><<<pgrid, GT_THREADS, 0, st>>>(pk, np, bk, range, g.nb, entries, later, o);
+    PJ_CUDA(cudaGetLastError());
+    if (nb > GT_LONG)
+        PJ_CUDA(launch_after(gt_probe_long_kernel<K, WIDE>, static_cast<unsigned>(sm_count()) * GT_LONG_CTAS, st, pk, np,
+                             bk, range, g.nb, entries, later, o));
+    PJ_CUDA(cudaGetLastError());
+    return PJ_OK;
 }
 
 template <typename K>
@@ -1092,33 +1134,9 @@ pj_status run_global(const pj_join_desc* d, const GlobalPlan& g, const Layout& L
         else
             gt_probe_kernel<K, 1><<<pgrid, GT_THREADS, 0, st>>>(pk, np, bk, table, g.nb, o);
     } else {
-        auto* counts = reinterpret_cast<uint32_t*>(ws + g.table);
-        auto* range = reinterpret_cast<uint2*>(ws + g.range);
-        auto* entries = reinterpret_cast<uint2*>(ws + g.entries);
-        // (the counter block's words double as 64-bit cursors: entries, and GtLong's)
-        auto* cursor = reinterpret_cast<unsigned long long*>(ws + L.counters);
-        if (small) {
-            gt_group_kernel<K><<<1, GT_GROUP_THREADS, 0, st>>>(bk, nb, g.nb, reinterpret_cast<uint32_t*>(ws),
-                                                               static_cast<int>(L.counters / 4) + 8, range, entries, cnt);
-        } else {
-            gt_count_kernel<K><<<bgrid, GT_THREADS, 0, st>>>(bk, nb, counts, g.nb, cnt);
-            PJ_CUDA(cudaGetLastError());
-            PJ_CUDA(launch_after(gt_alloc_kernel, (g.nb + GT_THREADS * GT_ALLOC - 1) / (GT_THREADS * GT_ALLOC), st, counts,
-                                 g.nb, range, cursor));
-            PJ_CUDA(launch_after(gt_place_kernel<K>, bgrid, st, bk, nb, range, g.nb, entries));
-        }
-        PJ_CUDA(cudaGetLastError());
-        for (int i = PJ_STAGE_BUILD_PASS2; i <= PJ_STAGE_JOIN; ++i) E.mark(i, st);
-        // (the list takes the counts' place: the ranges hold them by now)
-        const GtLong later = long_ranges(d->n_build, d->n_probe, d->key_bytes, cursor + 1, counts);
-        // (not launched ahead: beside the kernel before it, its CTAs would crowd on the few SMs that one leaves free --
-        // 2^16 x 2^14 4-byte rows, 16 a key, behind other work: 163 us, 48 with an SM each)
-        gt_probe_multi_kernel<K><<<pgrid, GT_THREADS, 0, st>>>(pk, np, bk, range, g.nb, entries, later, o);
-        PJ_CUDA(cudaGetLastError());
-        if (nb > GT_LONG) {
-            PJ_CUDA(launch_after(gt_probe_long_kernel<K>, static_cast<unsigned>(sm_count()) * GT_LONG_CTAS, st, pk, np, bk,
-                                 range, g.nb, entries, later, o));
-        }
+        if constexpr (sizeof(K) == 8)
+            if (g.wide) return run_global_repeated<K, true>(d, g, L, ws, o, st, E);
+        return run_global_repeated<K, false>(d, g, L, ws, o, st, E);
     }
     PJ_CUDA(cudaGetLastError());
     return PJ_OK;

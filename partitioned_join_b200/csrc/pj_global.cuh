@@ -19,8 +19,8 @@
 //     rows/s where 64-bit ones insert 61 G/s.
 //
 // Repeated build keys: rows grouped by bucket (count, allocate, place),
-// 8-byte entries {murmur(key), row} and each bucket's range; a lookup walks
-// its bucket.  Long buckets are left to a second launch, which cuts them into
+// entries {murmur(key), row} or, of 8-byte keys, {key, row}, and each bucket's
+// range; a lookup walks its bucket.  Long buckets are left to a second launch, which cuts them into
 // slices over the whole GPU, whatever probe rows meet them.
 //
 // Reference counterpart: hash_join (hash_join_kernels.cuh:24-200), which
@@ -46,17 +46,18 @@ constexpr uint32_t GT_SLICE = 32 * GT_SLICE_U;  // entries of a slice's step
 constexpr int GT_SLICES = 4;                // slices of a warp in flight together
 constexpr uint32_t GT_ROUND = GT_THREADS / 32 * GT_SLICES;  // slices of a CTA's round
 // From GT_WALK_PROBE probe rows on, whose tiles fill the GPU, the finder's warp
-// walks ranges of up to GT_WALK entries: 2^20 4-byte probe rows of ranges of
-// 256 take 660 us walked and 815 cut, 2^18 rows 245 and 238.  With 8-byte keys a
-// walk waits for a build key at every step (2400 us and 1536), but where few
-// rows of a warp meet a short range, a cut spends a whole round on them (2^21
-// rows, runs of 24 rows a key: 1354 us walked, 1535 cut; 96 rows: 1844 and 1951).
-constexpr int64_t GT_WALK_PROBE = int64_t(1) << 19;
+// walks ranges of up to GT_WALK entries (runs of 96 4-byte rows a key, 2^16
+// probe rows: 93 us walked, 50 cut; 2^18: 112 and 126; 2^20: 304 and 421; of
+// 600 rows 2^20: 1340 and 1900).  Entries that hold an 8-byte key are twice the
+// size (2^20 probe rows, runs of 96: 407 and 499; 256: 847 and 892; 600: 1943 and
+// 1982); those that do not are cut, since a walk waits for a build key at every
+// step (2^20 x 2^19 rows, runs of 40: 312 and 255; 256: 1287 and 878).
+constexpr int64_t GT_WALK_PROBE = int64_t(1) << 18;
 constexpr uint32_t GT_WALK_32 = 1024, GT_WALK_64 = 256;
 constexpr unsigned GT_LONG_CTAS = 4;        // CTAs per SM of the launch for them
 constexpr int GT_ROW_BITS = 22;             // 8-byte keys: row bits of a slot
 constexpr int64_t GT_MAX_BUILD = int64_t(1) << GT_ROW_BITS;  // build rows of a table
-constexpr int GT_STAGE = 2048;              // repeated keys: pairs a CTA stages for whole-run stores
+constexpr uint32_t GT_STAGE = 256;          // repeated keys: pairs a warp stages for whole-run stores
 
 struct GlobalOut {
     int32_t* out_build;  // nullptr: count only
@@ -419,7 +420,8 @@ __global__ void __launch_bounds__(GT_THREADS, STEPS == 1 ? 2048 / GT_THREADS : 1
 // A kernel of the chain below: the next one may be put in place, and this one
 // goes on when the one before has ended and its writes are visible.  (What
 // that one wrote is read by plain loads: a non-coherent load wants memory that
-// nobody writes while its kernel is there, and it may be there by then.)
+// nobody writes while its kernel is there, and one put in place ahead is there
+// by then; gt_probe_multi_kernel, which is not, reads entries by such loads.)
 __device__ __forceinline__ void gt_wait_before()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -433,7 +435,61 @@ __device__ __forceinline__ uint2 gt_load(const uint2* p)
     return v;
 }
 
+// One sector of entries: those at p and after it.
+__device__ __forceinline__ void gt_load_sector(const uint2* p, uint2 (&e)[4])
+{
+    uint32_t w[8];
+    gt_load_bucket(reinterpret_cast<const uint32_t*>(p), 0, w);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) e[v] = make_uint2(w[2 * v], w[2 * v + 1]);
+}
+__device__ __forceinline__ void gt_load_sector(const uint4* p, uint4 (&e)[2])
+{
+    uint32_t w[8];
+    gt_load_bucket(reinterpret_cast<const uint32_t*>(p), 0, w);
+#pragma unroll
+    for (int v = 0; v < 2; ++v) e[v] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+}
+
+__device__ __forceinline__ uint4 gt_load(const uint4* p)
+{
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // ---- repeated build keys ---------------------------------------------------
+
+// One build row among those of its bucket.  Narrow: {hash, row}; an equal hash
+// of an 8-byte key is compared with the build key, read from its column.  Wide
+// (8-byte keys): {key, row}, which saves a random sector a pair where the probe
+// side is no smaller than the build side (2^20 x 2^24 rows, four a key: 802 ->
+// 681 us by itself).
+template <typename K, bool WIDE> struct GtEntry {
+    using T = uint2;
+    static constexpr uint32_t SECTOR = 4;  // entries of 32 bytes
+    __device__ __forceinline__ static T make(uint32_t h, K, uint32_t row) { return make_uint2(h, row); }
+    __device__ __forceinline__ static T none(uint32_t h, K) { return make_uint2(~h, 0u); }  // equal to no such key
+    __device__ __forceinline__ static uint32_t row(const T& e) { return e.y; }
+    __device__ __forceinline__ static bool equal(const T& e, uint32_t h, K key, const K* __restrict__ bkeys)
+    {
+        return e.x == h && (sizeof(K) == 4 || bkeys[e.y] == key);
+    }
+};
+template <> struct GtEntry<int64_t, true> {
+    using T = uint4;
+    static constexpr uint32_t SECTOR = 2;
+    __device__ __forceinline__ static T make(uint32_t, int64_t key, uint32_t row)
+    {
+        return make_uint4(static_cast<uint32_t>(key), static_cast<uint32_t>(key >> 32), row, 0u);
+    }
+    __device__ __forceinline__ static T none(uint32_t, int64_t key) { return make(0u, ~key, 0u); }
+    __device__ __forceinline__ static uint32_t row(const T& e) { return e.z; }
+    __device__ __forceinline__ static bool equal(const T& e, uint32_t, int64_t key, const int64_t* __restrict__)
+    {
+        return e.x == static_cast<uint32_t>(key) && e.y == static_cast<uint32_t>(key >> 32);
+    }
+};
 
 template <typename K>
 __global__ void __launch_bounds__(GT_THREADS) gt_count_kernel(const K* __restrict__ keys, uint32_t n,
@@ -471,15 +527,17 @@ static __global__ void __launch_bounds__(GT_THREADS) gt_alloc_kernel(const uint3
 }
 
 // range[b].y moves from the bucket's start to its end
-template <typename K>
+template <typename K, bool WIDE>
 __global__ void __launch_bounds__(GT_THREADS) gt_place_kernel(const K* __restrict__ keys, uint32_t n, uint2* range,
-                                                              uint32_t nb, uint2* __restrict__ entries)
+                                                              uint32_t nb,
+                                                              typename GtEntry<K, WIDE>::T* __restrict__ entries)
 {
     gt_wait_before();
     const uint32_t i = blockIdx.x * GT_THREADS + threadIdx.x;
     if (i >= n) return;
-    const uint32_t h = hash_key(keys[i]);
-    entries[atomicAdd(&range[gt_bucket(h, nb)].y, 1u)] = make_uint2(h, i);
+    const K key = keys[i];
+    const uint32_t h = hash_key(key);
+    entries[atomicAdd(&range[gt_bucket(h, nb)].y, 1u)] = GtEntry<K, WIDE>::make(h, key, i);
 }
 
 // Count, allocate and place by one CTA, the buckets' counts in shared memory,
@@ -487,18 +545,17 @@ __global__ void __launch_bounds__(GT_THREADS) gt_place_kernel(const K* __restric
 // of up to GT_GROUP rows, whose joins wait for launches.
 constexpr int GT_GROUP_THREADS = 1024;
 constexpr int64_t GT_GROUP = 4096;
-template <typename K>
+template <typename K, bool WIDE>
 __global__ void __launch_bounds__(GT_GROUP_THREADS) gt_group_kernel(const K* __restrict__ keys, uint32_t n,
                                                                     uint32_t nb, uint32_t* head, int head_words,
                                                                     uint2* __restrict__ range,
-                                                                    uint2* __restrict__ entries,
+                                                                    typename GtEntry<K, WIDE>::T* __restrict__ entries,
                                                                     unsigned long long* count)
 {
     constexpr int U = 4;  // rows of a thread in flight
     constexpr uint32_t T = GT_GROUP_THREADS;
     __shared__ uint32_t s_at[GT_GROUP];  // counts, then places
     __shared__ uint32_t s_warp[32];
-    gt_wait_before();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t b = threadIdx.x; b < nb; b += T) s_at[b] = 0u;
     for (int i = threadIdx.x; i < head_words; i += T) head[i] = 0u;
@@ -510,11 +567,11 @@ __global__ void __launch_bounds__(GT_GROUP_THREADS) gt_group_kernel(const K* __r
             for (int u = 0; u < U; ++u) k[u] = i0 + u * T < n ? keys[i0 + u * T] : K(0);
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (i0 + u * T < n) f(i0 + u * T, hash_key(k[u]));
+                if (i0 + u * T < n) f(i0 + u * T, k[u], hash_key(k[u]));
         }
     };
     __syncthreads();
-    each([&](uint32_t, uint32_t h) { atomicAdd(&s_at[gt_bucket(h, nb)], 1u); });
+    each([&](uint32_t, K, uint32_t h) { atomicAdd(&s_at[gt_bucket(h, nb)], 1u); });
     __syncthreads();
     // (an odd run: the lanes walk 32 banks)
     const uint32_t run = ((nb + T - 1) / T) | 1u, b0 = threadIdx.x * run, b1 = min(b0 + run, nb);
@@ -536,7 +593,9 @@ __global__ void __launch_bounds__(GT_GROUP_THREADS) gt_group_kernel(const K* __r
         at += c;
     }
     __syncthreads();
-    each([&](uint32_t i, uint32_t h) { entries[atomicAdd(&s_at[gt_bucket(h, nb)], 1u)] = make_uint2(h, i); });
+    each([&](uint32_t i, K key, uint32_t h) {
+        entries[atomicAdd(&s_at[gt_bucket(h, nb)], 1u)] = GtEntry<K, WIDE>::make(h, key, i);
+    });
 }
 
 // Probe rows that meet a long range, for gt_probe_long_kernel: one word per
@@ -554,33 +613,31 @@ struct GtLong {
     }
 };
 
-template <typename K>
-__device__ __forceinline__ bool gt_equal(const uint2& e, uint32_t h, K key, const K* __restrict__ bkeys)
-{
-    return e.x == h && (sizeof(K) == 4 || bkeys[e.y] == key);
-}
-
-// Probe of the grouped rows: a counting walk, then a writing walk at the
-// positions it gave (the entries are in L1 by then).  A CTA's pairs pass
-// through shared memory so that they leave as whole runs: single pairs
-// stored by their finders were L2-request bound (4 M probe rows, 9.6 M
-// pairs: 170 us).
-template <typename K>
-__global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __restrict__ pkeys, uint32_t n,
-                                                                    const K* __restrict__ bkeys,
-                                                                    const uint2* range, uint32_t nb,
-                                                                    const uint2* entries, GtLong later,
-                                                                    GlobalOut o)
+// Probe of the grouped rows, bound by the latency of its loads (key, range,
+// entries).  A range is read in whole sectors, both rows of a lane together:
+// entry by entry a lane came back to its L1 line several times, and the lines of
+// 1300 lanes evict each other before it does (2^20 x 2^24 rows, 16 a key: 2.07 ->
+// 1.52 ms; a larger stage, which leaves less L1, 2.35).  A warp's pairs pass
+// through shared memory, so that they leave in runs of 256 however many a row
+// has; with 2048 staged a CTA, what did not fit was stored by its finders (the
+// same join 5.46 ms; four rows a key 585 -> 366 us).  Wide entries need 64
+// registers: five CTAs an SM would spill them (2^20 x 2^24, 4 a key: 466 -> 554);
+// narrow ones have 44 or 48 (six CTAs of 40: 366 -> 380).
+template <typename K, bool WIDE>
+__global__ void __launch_bounds__(GT_THREADS, WIDE ? 4 : 5)
+    gt_probe_multi_kernel(const K* __restrict__ pkeys, uint32_t n, const K* __restrict__ bkeys, const uint2* range,
+                          uint32_t nb, const typename GtEntry<K, WIDE>::T* entries, GtLong later, GlobalOut o)
 {
     __shared__ unsigned long long s_warp[GT_THREADS / 32 + 2];
-    __shared__ uint2 s_pair[GT_STAGE];
+    __shared__ uint2 s_pair[GT_THREADS / 32][GT_STAGE];
+    using E = GtEntry<K, WIDE>;
     gt_wait_before();
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t row0 = blockIdx.x * GT_TILE + threadIdx.x * GT_U;
     K k[GT_U];
-    uint32_t h[GT_U], lo[GT_U], hi[GT_U], c[GT_U];
-    uint32_t hit[GT_U];  // entries of a short range that match
+    uint32_t h[GT_U], lo[GT_U], hi[GT_U];
+    uint2* stage = s_pair[threadIdx.x >> 5];
     gt_load_pair<K>(pkeys, true, n, row0, k);
     uint32_t slices = 0;
 #pragma unroll
@@ -600,74 +657,120 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
         const unsigned long long unit = row0 / (32 * GT_U);
         later.list[at >> later.round_bits] = (unit << later.round_bits) | (at & ((1ull << later.round_bits) - 1ull));
     }
-    unsigned long long mine = 0;
+    // The walk of the short ranges, sector by sector: the pairs go to the warp's
+    // stage while it has room, a bit of hit[u] stands for one that did not fit.
+    constexpr uint32_t S = E::SECTOR;
+    const bool write = o.out_build != nullptr;
+    uint32_t staged = 0, at0[GT_U], hit[GT_U], span[GT_U], longest = 0;
 #pragma unroll
     for (int u = 0; u < GT_U; ++u) {
-        c[u] = 0;
-        const bool is_long = hi[u] - lo[u] > GT_LONG;
+        at0[u] = lo[u] & ~(S - 1u);
+        span[u] = hi[u] == lo[u] || hi[u] - at0[u] > GT_LONG ? 0u : hi[u] - at0[u];
+        longest = max(longest, span[u]);
         hit[u] = 0;
-        if (!is_long) {
-            for (uint32_t i = lo[u]; i < hi[u]; i += GT_WALK_U) {
-                uint2 e[GT_WALK_U];
-                bool eq[GT_WALK_U];
-#pragma unroll
-                for (int v = 0; v < GT_WALK_U; ++v) e[v] = i + v < hi[u] ? gt_load(entries + i + v) : make_uint2(~h[u], 0u);
-#pragma unroll
-                for (int v = 0; v < GT_WALK_U; ++v) eq[v] = gt_equal<K>(e[v], h[u], k[u], bkeys);
-#pragma unroll
-                for (int v = 0; v < GT_WALK_U; ++v) hit[u] |= eq[v] ? 1u << (i - lo[u] + v) : 0u;
-            }
-            c[u] = __popc(hit[u]);
-        }
-        for (uint32_t todo = __ballot_sync(0xffffffffu, is_long); todo; todo &= todo - 1u) {
-            const int owner = __ffs(todo) - 1;
-            const uint32_t a = __shfl_sync(0xffffffffu, lo[u], owner), z = __shfl_sync(0xffffffffu, hi[u], owner);
-            const uint32_t hh = __shfl_sync(0xffffffffu, h[u], owner);
-            const K kk = __shfl_sync(0xffffffffu, k[u], owner);
-            uint32_t found = 0;
-            for (uint32_t i = a + lane; i < z; i += 32) found += gt_equal<K>(gt_load(entries + i), hh, kk, bkeys) ? 1u : 0u;
-            found = __reduce_add_sync(0xffffffffu, found);
-            if (lane == owner) c[u] = found;
-        }
-        mine += c[u];
     }
-    unsigned long long pos = gt_reserve(mine, s_warp, o.count);
-    if (o.out_build == nullptr) return;
-    const unsigned long long first = s_warp[GT_THREADS / 32], all = s_warp[GT_THREADS / 32 + 1];
-    const bool staged = all <= GT_STAGE;
-    auto put = [&](unsigned long long at, uint32_t b, uint32_t q) {
-        if (staged) s_pair[at - first] = make_uint2(b, q);
-        else gt_store_pair(o, at, static_cast<int32_t>(b), q);
-    };
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    for (uint32_t i = 0; i < longest; i += GT_WALK_U) {
+        typename E::T e[GT_U][GT_WALK_U / S][S];
+        bool eq[GT_U][GT_WALK_U];
+#pragma unroll
+        for (int u = 0; u < GT_U; ++u)
+#pragma unroll
+            for (uint32_t v = 0; v < GT_WALK_U; v += S)
+                if (i + v < span[u]) gt_load_sector(entries + at0[u] + i + v, e[u][v / S]);
+#pragma unroll
+        for (int u = 0; u < GT_U; ++u)
+#pragma unroll
+            for (uint32_t v = 0; v < GT_WALK_U; ++v)
+                eq[u][v] = i + v < span[u] && at0[u] + i + v >= lo[u] && E::equal(e[u][v / S][v % S], h[u], k[u], bkeys);
+#pragma unroll
+        for (int u = 0; u < GT_U; ++u)
+#pragma unroll
+            for (uint32_t v = 0; v < GT_WALK_U; ++v) {
+                const uint32_t bal = __ballot_sync(0xffffffffu, eq[u][v]), n_eq = __popc(bal);
+                if (!write) {
+                    staged += n_eq;
+                } else if (staged + n_eq <= GT_STAGE) {
+                    if (eq[u][v]) stage[staged + __popc(bal & lt)] = make_uint2(E::row(e[u][v / S][v % S]), row0 + u);
+                    staged += n_eq;
+                } else if (eq[u][v]) {
+                    hit[u] |= 1u << (i + v);
+                }
+            }
+    }
+    // the longer ones, counted by the whole warp
+    uint32_t more = 0;
 #pragma unroll
     for (int u = 0; u < GT_U; ++u) {
-        const bool is_long = hi[u] - lo[u] > GT_LONG;
-        for (uint32_t m = hit[u]; m; m &= m - 1u) put(pos++, gt_load(entries + lo[u] + __ffs(m) - 1).y, row0 + u);
-        for (uint32_t todo = __ballot_sync(0xffffffffu, is_long && c[u] > 0); todo; todo &= todo - 1u) {
+        more += __popc(hit[u]);
+        uint32_t found = 0;  // this lane's row of them
+        for (uint32_t todo = __ballot_sync(0xffffffffu, hi[u] - at0[u] > GT_LONG && hi[u] != lo[u]); todo; todo &= todo - 1u) {
             const int owner = __ffs(todo) - 1;
             const uint32_t a = __shfl_sync(0xffffffffu, lo[u], owner), z = __shfl_sync(0xffffffffu, hi[u], owner);
             const uint32_t hh = __shfl_sync(0xffffffffu, h[u], owner);
-            const uint32_t r = __shfl_sync(0xffffffffu, row0 + u, owner);
             const K kk = __shfl_sync(0xffffffffu, k[u], owner);
-            unsigned long long at = __shfl_sync(0xffffffffu, pos, owner);
-            for (uint32_t i0 = a; i0 < z; i0 += 32) {
-                const uint32_t i = i0 + lane;
-                uint2 e = make_uint2(0u, 0u);
-                if (i < z) e = gt_load(entries + i);
-                const bool hit = i < z && gt_equal<K>(e, hh, kk, bkeys);
-                const uint32_t bal = __ballot_sync(0xffffffffu, hit);
-                if (hit) put(at + __popc(bal & lt), e.y, r);
-                at += __popc(bal);
+            uint32_t n_eq = 0;
+            for (uint32_t i = a + lane; i < z; i += 64) {
+                const typename E::T e0 = gt_load(entries + i);
+                const typename E::T e1 = i + 32 < z ? gt_load(entries + i + 32) : E::none(hh, kk);
+                n_eq += (E::equal(e0, hh, kk, bkeys) ? 1u : 0u) + (E::equal(e1, hh, kk, bkeys) ? 1u : 0u);
             }
-            if (lane == owner) pos = at;
+            n_eq = __reduce_add_sync(0xffffffffu, n_eq);
+            if (lane == owner) found = n_eq;
+        }
+        if (found == 0) hi[u] = lo[u];  // (no second walk)
+        more += found;
+    }
+    more = __reduce_add_sync(0xffffffffu, more);
+    // lane 31 speaks for the warp: its position is the warp's base
+    const unsigned long long at = gt_reserve(lane == 31 ? staged + more : 0u, s_warp, o.count);
+    unsigned long long pos = __shfl_sync(0xffffffffu, at, 31);
+    if (!write) return;
+    auto leave = [&]() {
+        __syncwarp();
+        for (uint32_t i = lane; i < staged; i += 32) {
+            const uint2 x = stage[i];
+            gt_store_pair(o, pos + i, static_cast<int32_t>(x.x), x.y);
+        }
+        pos += staged;
+        staged = 0;
+        __syncwarp();
+    };
+    leave();
+    if (more == 0) return;
+    auto put = [&](bool has, uint32_t b, uint32_t q) {
+        const uint32_t bal = __ballot_sync(0xffffffffu, has);
+        if (has) stage[staged + __popc(bal & lt)] = make_uint2(b, q);
+        staged += __popc(bal);
+        if (staged > GT_STAGE - 32) leave();
+    };
+    while (__any_sync(0xffffffffu, (hit[0] | hit[1]) != 0u)) {
+        const int u = hit[0] ? 0 : 1;
+        const uint32_t m = u == 0 ? hit[0] : hit[1];
+        uint32_t b = 0;
+        if (m) b = E::row(gt_load(entries + (u == 0 ? at0[0] : at0[1]) + __ffs(m) - 1));
+        put(m != 0u, b, row0 + u);
+        if (u == 0) hit[0] = m & (m - 1u);
+        else hit[1] = m & (m - 1u);
+    }
+#pragma unroll
+    for (int u = 0; u < GT_U; ++u) {
+        for (uint32_t todo = __ballot_sync(0xffffffffu, hi[u] - at0[u] > GT_LONG && hi[u] != lo[u]); todo; todo &= todo - 1u) {
+            const int owner = __ffs(todo) - 1;
+            const uint32_t a = __shfl_sync(0xffffffffu, lo[u], owner), z = __shfl_sync(0xffffffffu, hi[u], owner);
+            const uint32_t hh = __shfl_sync(0xffffffffu, h[u], owner);
+            const uint32_t q = __shfl_sync(0xffffffffu, row0 + u, owner);
+            const K kk = __shfl_sync(0xffffffffu, k[u], owner);
+            for (uint32_t i0 = a; i0 < z; i0 += 64) {
+                const uint32_t i = i0 + lane;
+                const typename E::T e0 = i < z ? gt_load(entries + i) : E::none(hh, kk);
+                const typename E::T e1 = i + 32 < z ? gt_load(entries + i + 32) : E::none(hh, kk);
+                put(E::equal(e0, hh, kk, bkeys), E::row(e0), q);
+                if (i0 + 32 < z) put(E::equal(e1, hh, kk, bkeys), E::row(e1), q);
+            }
         }
     }
-    if (!staged) return;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < static_cast<uint32_t>(all); i += GT_THREADS) {
-        const uint2 p = s_pair[i];
-        gt_store_pair(o, first + i, static_cast<int32_t>(p.x), p.y);
-    }
+    leave();
 }
 
 // The probe rows that gt_probe_multi_kernel left: the rounds of all words, in
@@ -676,13 +779,14 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_multi_kernel(const K* __r
 // store, so a range is walked once, and the pairs of a round leave in whole
 // runs at a position reserved by one atomic.  (Walked by one warp a row,
 // 64 probe rows of a key with 2^20 build rows took 1.27 s.)
-template <typename K>
+template <typename K, bool WIDE>
 __global__ void __launch_bounds__(GT_THREADS) gt_probe_long_kernel(const K* __restrict__ pkeys, uint32_t n,
                                                                    const K* __restrict__ bkeys,
                                                                    const uint2* range, uint32_t nb,
-                                                                   const uint2* entries, GtLong later,
+                                                                   const typename GtEntry<K, WIDE>::T* entries, GtLong later,
                                                                    GlobalOut o)
 {
+    using E = GtEntry<K, WIDE>;
     constexpr uint32_t ROWS = 32 * GT_U;  // probe rows of a word
     static_assert(ROWS == 64, "two rows a lane");
     constexpr int NW = GT_THREADS / 32;
@@ -759,20 +863,20 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_long_kernel(const K* __re
                 hi[t] = part < later.slices(to - from) ? min(lo[t] + later.slice, to) : 0u;
             }
             for (uint32_t step = 0; step < later.slice; step += GT_SLICE, buffer ^= 1) {
-                uint2 e[GT_SLICES][GT_SLICE_U];
+                typename E::T e[GT_SLICES][GT_SLICE_U];
 #pragma unroll
                 for (int t = 0; t < GT_SLICES; ++t)
 #pragma unroll
                     for (int v = 0; v < GT_SLICE_U; ++v) {
                         const uint32_t i = lo[t] + step + v * 32 + lane;
-                        e[t][v] = i < hi[t] ? gt_load(entries + i) : make_uint2(~s_hash[row[t]], 0u);
+                        e[t][v] = i < hi[t] ? gt_load(entries + i) : E::none(s_hash[row[t]], s_key[row[t]]);
                     }
                 uint32_t off[GT_SLICES][GT_SLICE_U], hits = 0, total = 0;
 #pragma unroll
                 for (int t = 0; t < GT_SLICES; ++t)
 #pragma unroll
                     for (int v = 0; v < GT_SLICE_U; ++v) {
-                        const bool hit = gt_equal<K>(e[t][v], s_hash[row[t]], s_key[row[t]], bkeys);
+                        const bool hit = E::equal(e[t][v], s_hash[row[t]], s_key[row[t]], bkeys);
                         const uint32_t bal = __ballot_sync(0xffffffffu, hit);
                         off[t][v] = total + __popc(bal & lt);
                         total += __popc(bal);
@@ -787,7 +891,7 @@ __global__ void __launch_bounds__(GT_THREADS) gt_probe_long_kernel(const K* __re
 #pragma unroll
                     for (int v = 0; v < GT_SLICE_U; ++v)
                         if (hits >> (t * GT_SLICE_U + v) & 1u)
-                            gt_store_pair(o, base + off[t][v], static_cast<int32_t>(e[t][v].y), row0 + row[t]);
+                            gt_store_pair(o, base + off[t][v], static_cast<int32_t>(E::row(e[t][v])), row0 + row[t]);
             }
         }
         ++w;
