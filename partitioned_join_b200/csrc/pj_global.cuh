@@ -617,12 +617,11 @@ struct GtLong {
 // entries).  A range is read in whole sectors, both rows of a lane together:
 // entry by entry a lane came back to its L1 line several times, and the lines of
 // 1300 lanes evict each other before it does (2^20 x 2^24 rows, 16 a key: 2.07 ->
-// 1.52 ms; a larger stage, which leaves less L1, 2.35).  A warp's pairs pass
+// 1.48 ms; a larger stage, which leaves less L1, 2.35).  A warp's pairs pass
 // through shared memory, so that they leave in runs of 256 however many a row
 // has; with 2048 staged a CTA, what did not fit was stored by its finders (the
-// same join 5.46 ms; four rows a key 585 -> 366 us).  Wide entries need 64
-// registers: five CTAs an SM would spill them (2^20 x 2^24, 4 a key: 466 -> 554);
-// narrow ones have 44 or 48 (six CTAs of 40: 366 -> 380).
+// same join 5.46 ms; four rows a key 585 -> 339 us).  Wide entries need 64
+// registers: five CTAs an SM would spill them (2^20 x 2^24, 4 a key: 466 -> 554).
 template <typename K, bool WIDE>
 __global__ void __launch_bounds__(GT_THREADS, WIDE ? 4 : 5)
     gt_probe_multi_kernel(const K* __restrict__ pkeys, uint32_t n, const K* __restrict__ bkeys, const uint2* range,
@@ -740,6 +739,11 @@ __global__ void __launch_bounds__(GT_THREADS, WIDE ? 4 : 5)
     if (more == 0) return;
     auto put = [&](bool has, uint32_t b, uint32_t q) {
         const uint32_t bal = __ballot_sync(0xffffffffu, has);
+        if (bal == 0xffffffffu) {  // a run by itself (2^20 x 2^22 rows, 64 a key: 849 -> 683 us)
+            gt_store_pair(o, pos + lane, static_cast<int32_t>(b), q);
+            pos += 32;
+            return;
+        }
         if (has) stage[staged + __popc(bal & lt)] = make_uint2(b, q);
         staged += __popc(bal);
         if (staged > GT_STAGE - 32) leave();
