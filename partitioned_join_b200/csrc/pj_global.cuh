@@ -47,11 +47,12 @@ constexpr int GT_SLICES = 4;                // slices of a warp in flight togeth
 constexpr uint32_t GT_ROUND = GT_THREADS / 32 * GT_SLICES;  // slices of a CTA's round
 // From GT_WALK_PROBE probe rows on, whose tiles fill the GPU, the finder's warp
 // walks ranges of up to GT_WALK entries (runs of 96 4-byte rows a key, 2^16
-// probe rows: 93 us walked, 50 cut; 2^18: 112 and 126; 2^20: 304 and 421; of
-// 600 rows 2^20: 1340 and 1900).  Entries that hold an 8-byte key are twice the
-// size (2^20 probe rows, runs of 96: 407 and 499; 256: 847 and 892; 600: 1943 and
-// 1982); those that do not are cut, since a walk waits for a build key at every
-// step (2^20 x 2^19 rows, runs of 40: 312 and 255; 256: 1287 and 878).
+// probe rows: 93 us walked, 50 cut; 2^18: 100 and 126; 2^20: 263 and 421; of
+// 600 rows 2^20: 1198 and 1900).  Entries that hold an 8-byte key are twice the
+// size (2^20 probe rows, runs of 96: 384 and 499; 256: 820 and 892; 600, before
+// whole runs were stored at once: 1943 and 1982); those that do not are cut, since
+// a walk waits for a build key at every step (2^20 x 2^19 rows, runs of 40: 312 and
+// 255; 256: 1287 and 878).
 constexpr int64_t GT_WALK_PROBE = int64_t(1) << 18;
 constexpr uint32_t GT_WALK_32 = 1024, GT_WALK_64 = 256;
 constexpr unsigned GT_LONG_CTAS = 4;        // CTAs per SM of the launch for them
